@@ -1,17 +1,16 @@
 // Object engine kernels (see engine.hpp). A "group" — one CTA, or a cluster of 4 or 8 CTAs
-// for a large object — runs one object's chain. Every frontier round has two steps separated by a
-// group barrier: step A stages each frontier voxel (flag cleared, distance read, neighbour mask),
-// step B spreads its 26 (voxel, neighbour) items densely over the threads, so that thousands of
-// independent relaxations are in flight at once. When every CTA's share of the frontier fits its
-// shared-memory staging, each CTA stages its own share there and runs only that share's items
-// (an item then reads its voxel's fields without an L2 round trip); larger frontiers are staged
-// in HBM and their items spread over the whole group. The group's counters live in the shared memory
-// of its first CTA (distributed shared memory for a cluster, updated with 32-bit atomics only);
-// 64-bit reductions (nearest rail, nearest deferred voxel, argmax) keep one copy per CTA, updated
-// with CTA-local atomics and combined across the group at barriers. State other threads update
-// with atomics (distances, keys, flags, staged entries) is always read through L2; state that is
-// only written between floods, behind a group barrier (PDRF during a railroad flood, liveness
-// during an invalidation), is read through L1, where a voxel's 26 neighbours find it again.
+// for a large object — runs one object's chain as floods of synchronised rounds. A round's frontier
+// is a queue of (voxel, value) pairs in the shared memory of the group's CTAs, each CTA taking an
+// even share of the whole; a warp takes a frontier voxel, its lanes the 26 neighbours, so that the
+// neighbour offsets and step weights are registers and pushes are aggregated by ballot. A pair is
+// stale when the voxel's value has moved on since it was queued, so a queue needs no membership
+// flags; what does not fit the queue spills to the object's list in HBM, kept unique by a flag.
+// The group's counters live in the shared memory of its first CTA (distributed shared memory for a
+// cluster, updated with 32-bit atomics only); 64-bit reductions (nearest rail, nearest deferred
+// voxel, argmax) keep one copy per CTA, updated with CTA-local atomics and combined across the group
+// at barriers. State other threads update with atomics (distances, keys, flags, lists) is always
+// read through L2; state that is only written between floods, behind a group barrier (PDRF during a
+// railroad flood), is read through L1, where a voxel's 26 neighbours find it again.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -29,23 +28,30 @@ namespace cg = cooperative_groups;
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr unsigned long long kMinFarNone = 0x7f8000007f800000ull;
-constexpr unsigned long long kClaimedMark = 0xFFFFFFFFFFFFFFFEull;
-// Resident engine CTAs per SM: 4 x 512 threads (full occupancy) at up to 32 registers each; the
-// spills this forces cost less than the latency the extra warps hide.
-constexpr int kEngineCtasPerSm = 4;
+// Invalidation keys (M bits << 32 | source + 1): 0 marks a dead voxel, below every offer. A voxel on
+// the waiting list holds its best offer with this bit (a distance's sign bit), which puts it above
+// every claim; BK_UNCLAIMED, above every offer, is a voxel at rest.
+constexpr unsigned long long kWaits = 1ull << 63;
 
 struct Shared {
   // the object (written by the group's first CTA, copied by the others)
   int obj, begin, count, status;
   int a0, sx, sy, sz;
+  // unsigned divisions by sx * sy and sx as multiplications (FastDiv)
+  unsigned mxy, mx;
+  int pxy, px;
   // group counters (used in the first CTA's copy)
-  int cnt[3];  // frontier counters, a ring: current = cnt[r % 3], next = cnt[(r + 1) % 3]
-  int n_far, n_keep, n_touch, flag, len;
-  float T;
+  int spilled[3];  // spilled frontier voxels, a ring like qn
+  int far_n[2];    // the two deferred lists' lengths
+  int n_touch, n_redo, len;
   unsigned long long rounds;
   // per-CTA copies, combined with Group::min_over / max_over
-  unsigned long long rb, minfar, best;
-  unsigned lowest, pos;
+  int qn[3];  // this CTA's queue, a ring: current = qn[r % 3], next = qn[(r + 1) % 3]
+  unsigned long long rb, minfar[2], best;
+  unsigned lowest[2], pos;
+  // each CTA's own result of a band end
+  int flag;
+  float T;
   // this CTA's copy of the object's neighbour offsets and step weights
   int off[26];
   float w[26];
@@ -73,13 +79,21 @@ __device__ __forceinline__ void unravel3(int i, int sx, int sy, int &x, int &y, 
   x = r - y * sx;
 }
 
-__device__ __forceinline__ unsigned long long pack3(int x, int y, int z) {
-  return (unsigned long long)x | ((unsigned long long)y << 21) | ((unsigned long long)z << 42);
+// n / d for 0 <= n < 2^31 as n * m >> p with p = 31 + ceil(log2 d) and m = ceil(2^p / d): m exceeds
+// 2^p / d by less than 1, so the product exceeds n 2^p / d by less than 2^31 <= 2^p / d.
+__device__ __forceinline__ void fast_div(unsigned d, unsigned &m, int &p) {
+  p = 31 + (d > 1 ? 32 - __clz(int(d - 1)) : 0);
+  m = unsigned(((1ull << p) + d - 1) / d);
 }
-__device__ __forceinline__ void unpack3(unsigned long long p, int &x, int &y, int &z) {
-  x = int(p & 0x1FFFFF);
-  y = int((p >> 21) & 0x1FFFFF);
-  z = int(p >> 42);
+__device__ __forceinline__ int divided(int n, unsigned m, int p) {
+  return int((static_cast<unsigned long long>(unsigned(n)) * m) >> p);
+}
+// The coordinates of the object's arena-local flat index i.
+__device__ __forceinline__ void coordinates(const Shared &sh, int i, int &x, int &y, int &z) {
+  z = divided(i, sh.mxy, sh.pxy);
+  const int r = i - z * (sh.sx * sh.sy);
+  y = divided(r, sh.mx, sh.px);
+  x = r - y * sh.sx;
 }
 
 // A group of C CTAs working on one object. For C == 1 it is the CTA.
@@ -144,30 +158,141 @@ __device__ __forceinline__ long long capped(const EngineArgs &a, long long bound
   return a.round_limit > 0 && a.round_limit < bound ? a.round_limit : bound;
 }
 
-// Per-CTA staging of a round's frontier in shared memory. When every CTA's share of the frontier
-// fits, a CTA stages its own share (step A) and spreads only that share's (voxel, neighbour) items
-// over its threads (step B): the items then read their voxel's staged fields from shared memory
-// instead of L2, which takes one to four dependent L2 round trips out of every item's chain.
-// Larger frontiers go through the global staging arrays, items spread over the whole group.
-constexpr int kStageBytes = 18432;
-constexpr int kFloodStage = kStageBytes / 12;  // distance|mask (8) + voxel (4)
-constexpr int kInvalStage = kStageBytes / 36;  // key (8) + both positions (16) + voxel, mask, reach (12)
-constexpr int kBandStage = kStageBytes / 24;   // best offer (8) + position (8) + voxel, mask (8)
+// The queues' shared memory. Floods: two buffers of (voxel, distance bits) pairs. Invalidation: two
+// buffers of (voxel, key) pairs and the round's staged records. Four resident CTAs per SM then leave
+// half of the SM's 256 KB to L1, which holds the penalties.
+constexpr int kQueueBytes = 28672;
+constexpr int kFloodQueue = kQueueBytes / 16;   // pairs per buffer
+constexpr int kInvalQueue = kQueueBytes / 56;   // pairs per buffer, and records
+constexpr int kPipe = 2;  // frontier voxels a warp has in flight: their loads overlap
 
-__device__ __forceinline__ unsigned char *stage_bytes() {
-  __shared__ __align__(16) unsigned char buf[kStageBytes];
+__device__ __forceinline__ unsigned char *queue_bytes() {
+  __shared__ __align__(16) unsigned char buf[kQueueBytes];
   return buf;
 }
 
-// This CTA's share [lo, hi) of n entries, when the largest share fits `cap` (the same answer in
-// every CTA of the group, which all read the same n).
+// This CTA's even share [lo, hi) of the entries that the group's CTAs hold in their queues, taken in
+// rank order (pre: before lane q's CTA). Every warp computes it; every CTA reads the same counts.
+struct Share {
+  int lo, hi, total, pre;
+};
+
 template <int C>
-__device__ __forceinline__ bool own_share(int n, int cap, int &lo, int &hi) {
-  if ((n + C - 1) / C > cap) return false;
-  const int r = Group<C>::rank();
-  lo = int((long long)n * r / C);
-  hi = int((long long)n * (r + 1) / C);
-  return true;
+__device__ __forceinline__ Share share_of(Shared &sh, int slot, int cap) {
+  Share s;
+  if constexpr (C == 1) {
+    s.lo = 0;
+    s.hi = s.total = min(vload(&sh.qn[slot]), cap);
+    s.pre = 0;
+  } else {
+    const int lane = threadIdx.x & 31;
+    const int n = lane < C ? min(vload(cg::this_cluster().map_shared_rank(&sh.qn[slot], lane)), cap) : 0;
+    int sum = n;
+#pragma unroll
+    for (int off = 1; off < C; off <<= 1) {
+      const int o = __shfl_up_sync(kFull, sum, off);
+      if (lane >= off) sum += o;
+    }
+    s.total = __shfl_sync(kFull, sum, C - 1);
+    s.pre = sum - n;
+    const int r = Group<C>::rank();
+    s.lo = s.total * r / C;
+    s.hi = s.total * (r + 1) / C;
+  }
+  return s;
+}
+
+// The CTA whose queue holds entry i of the group's, and the entry's place there (i may differ
+// between lanes; every lane calls).
+template <int C>
+__device__ __forceinline__ void locate(const Share &s, int i, int &rank, int &at) {
+  rank = 0;
+  at = i;
+  if constexpr (C > 1) {
+#pragma unroll
+    for (int q = 1; q < C; ++q) {
+      const int p = __shfl_sync(kFull, s.pre, q);
+      if (p <= i) { rank = q; at = i - p; }
+    }
+  }
+}
+
+// p of the group's first CTA r's copy.
+template <int C, class T>
+__device__ __forceinline__ T *of_rank(T *p, int r) {
+  if constexpr (C == 1) return p;
+  else return cg::this_cluster().map_shared_rank(p, r);
+}
+
+__device__ __forceinline__ unsigned below(int lane) { return (1u << lane) - 1u; }
+
+// Appends v of the lanes with p to a list whose length is *count (every lane of the warp calls).
+__device__ __forceinline__ void append(bool p, int v, int *list, int *count) {
+  const unsigned b = __ballot_sync(kFull, p);
+  if (!b) return;
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(count, __popc(b));
+  base = __shfl_sync(kFull, base, 0);
+  if (p) list[base + __popc(b & below(lane))] = v;
+}
+
+// Places in this CTA's queue `slot` and in two of the object's lists for what the lanes of a warp push
+// out of kPipe voxels' neighbourhoods: one counter atomic per list, the three at once, since each is a
+// round trip (to the group's first CTA for the lists).
+struct Places {
+  int queue, touched, far;  // each list's next place; take() hands them out voxel by voxel
+  __device__ static int take(int &next, bool p) {
+    const unsigned b = __ballot_sync(kFull, p);
+    const int at = next + __popc(b & below(threadIdx.x & 31));
+    next += __popc(b);
+    return at;
+  }
+};
+
+__device__ __forceinline__ Places reserve(const bool (&queued)[kPipe], const bool (&touched)[kPipe],
+                                          const bool (&far)[kPipe], int *queue_n, int *touched_n, int *far_n) {
+  const int lane = threadIdx.x & 31;
+  int nq = 0, nt = 0, nf = 0;
+#pragma unroll
+  for (int j = 0; j < kPipe; ++j) {
+    nq += __popc(__ballot_sync(kFull, queued[j]));
+    nt += __popc(__ballot_sync(kFull, touched[j]));
+    nf += __popc(__ballot_sync(kFull, far[j]));
+  }
+  const int n = lane == 0 ? nq : lane == 1 ? nt : lane == 2 ? nf : 0;
+  int base = 0;
+  if (n) base = atomicAdd(lane == 0 ? queue_n : lane == 1 ? touched_n : far_n, n);
+  return {__shfl_sync(kFull, base, 0), __shfl_sync(kFull, base, 1), __shfl_sync(kFull, base, 2)};
+}
+
+// A place in this CTA's next queue for each lane with p (at or past the queue's end: spill).
+__device__ __forceinline__ int queue_place(Shared &sh, bool p, unsigned b, int slot) {
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(&sh.qn[slot], __popc(b));
+  base = __shfl_sync(kFull, base, 0);
+  return base + __popc(b & below(lane));
+}
+
+// A voxel that found no place in a queue goes to the round's spill list unless `bit` says it is there.
+__device__ __forceinline__ void spill(const EngineArgs &a, int v, unsigned bit, int *list, int *count) {
+  if (!(atomicOr(a.flags + v, bit) & bit)) list[atomicAdd(count, 1)] = v;
+}
+// The flag of the spill list that round r reads: two, so that round r clears its own while it sets
+// the other for the round after.
+__device__ __forceinline__ unsigned spill_bit(int r) { return (r & 1) ? kSpillOdd : kSpillEven; }
+
+// Queues (v, d) of the lanes with p for round r + 1 of a flood.
+__device__ __forceinline__ void queue_flood(const EngineArgs &a, Shared &sh, Shared *L, bool p, int v, unsigned d, int r,
+                                            int *spill_list) {
+  const unsigned b = __ballot_sync(kFull, p);
+  if (!b) return;
+  const int slot = (r + 1) % 3;
+  const int at = queue_place(sh, p, b, slot);
+  if (!p) return;
+  if (at < kFloodQueue) reinterpret_cast<uint2 *>(queue_bytes())[((r + 1) & 1) * kFloodQueue + at] = make_uint2(unsigned(v), d);
+  else spill(a, v, spill_bit(r + 1), spill_list, &L->spilled[slot]);
 }
 
 // Pulls the next object for this group; false when its queue is empty. The group's first CTA
@@ -197,6 +322,8 @@ __device__ bool next_object(const EngineArgs &a, Shared &sh, Shared *L, bool big
     if (sh.obj >= 0) {
       sh.begin = vload(&L->begin); sh.count = vload(&L->count);
       sh.a0 = vload(&L->a0); sh.sx = vload(&L->sx); sh.sy = vload(&L->sy); sh.sz = vload(&L->sz);
+      fast_div(unsigned(sh.sx) * unsigned(sh.sy), sh.mxy, sh.pxy);
+      fast_div(unsigned(sh.sx), sh.mx, sh.px);
     }
   }
   __syncthreads();
@@ -238,79 +365,107 @@ __device__ float freespace_seed(const EngineArgs &a, int x, int y, int z, int rx
 
 // seed_radius > 0 (a soma's DAF): every object voxel within it of `source` starts at its
 // free-space seed, and the rounds relax from all of them.
+// A round waits for two dependent L2 round trips (the neighbours' distances, then the atomic
+// minimum of those that improve) and one group barrier. A queued pair whose voxel has a smaller
+// distance by now is skipped: that distance has been queued too.
 template <int C>
 __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, float *d, int source, int *A, int *B,
-                                unsigned long long *wide, float seed_radius = 0.0f) {
+                                float seed_radius = 0.0f) {
   using G = Group<C>;
-  if (G::first()) { L->cnt[0] = 0; L->cnt[1] = 0; L->cnt[2] = 0; }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  if (threadIdx.x == 0) { sh.qn[0] = 0; sh.qn[1] = 0; sh.qn[2] = 0; }
+  if (G::first()) { L->spilled[0] = 0; L->spilled[1] = 0; L->spilled[2] = 0; }
   G::sync();
+  uint2 *queue = reinterpret_cast<uint2 *>(queue_bytes());
+  int r = -1;  // the seeds are queued for round 0
   if (seed_radius > 0.0f) {
     int rx, ry, rz;
     unravel3(source - sh.a0, sh.sx, sh.sy, rx, ry, rz);
-    for (int i = G::tid(); i < sh.count; i += G::threads()) {
-      const int v = a.vox[sh.begin + i];
-      int x, y, z;
-      unravel3(v - sh.a0, sh.sx, sh.sy, x, y, z);
-      const float s = freespace_seed(a, x, y, z, rx, ry, rz, seed_radius);
-      if (s < 0.0f) continue;
-      d[v] = s;
-      atomicOr(a.flags + v, kNearQueued);
-      A[atomicAdd(&L->cnt[0], 1)] = v;
+    for (int i0 = G::tid() - lane; i0 < sh.count; i0 += G::threads()) {
+      const int i = i0 + lane;
+      float s = -1.0f;
+      int v = 0;
+      if (i < sh.count) {
+        v = a.vox[sh.begin + i];
+        int x, y, z;
+        unravel3(v - sh.a0, sh.sx, sh.sy, x, y, z);
+        s = freespace_seed(a, x, y, z, rx, ry, rz, seed_radius);
+        if (s >= 0.0f) d[v] = s;
+      }
+      queue_flood(a, sh, L, s >= 0.0f, v, __float_as_uint(s), r, A);
     }
   } else if (G::first()) {
     d[source] = 0.0f;
-    atomicOr(a.flags + source, kNearQueued);
-    A[0] = source;
-    L->cnt[0] = 1;
+    queue[0] = make_uint2(unsigned(source), 0u);
+    sh.qn[0] = 1;
   }
   G::sync();
+  const bool neighbour = lane < 26;
+  const int off = neighbour ? sh.off[lane] : 0;
+  const float w = neighbour ? sh.w[lane] : 0.0f;
   const long long bound = capped(a, 8LL * sh.count + 256);
-  for (int r = 0;; ++r) {
-    int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
-    const int nc = vload(&L->cnt[r % 3]);
-    if (nc == 0) break;
+  for (r = 0;; ++r) {
+    const Share s = share_of<C>(sh, r % 3, kFloodQueue);
+    const int spilled = vload(&L->spilled[r % 3]);
+    if (s.total + spilled == 0) break;
     if (r >= bound) return false;
-    if (G::first()) L->cnt[(r + 2) % 3] = 0;
-    int *next_count = &L->cnt[(r + 1) % 3];
-    auto relax = [&](unsigned long long e, int u, int k) {
-      if (!((unsigned(e) >> k) & 1u)) return;
-      const int v = u + sh.off[k];
-      const float cand = __fadd_rn(__uint_as_float(unsigned(e >> 32)), sh.w[k]);
-      const float old = atomic_min_pos(d + v, cand);
-      if (old > cand && !(atomicOr(a.flags + v, kNearQueued) & kNearQueued)) nxt[atomicAdd(next_count, 1)] = v;
+    if (threadIdx.x == 0) sh.qn[(r + 2) % 3] = 0;
+    if (G::first()) L->spilled[(r + 2) % 3] = 0;
+    int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
+    auto relax = [&](const uint2 (&e)[kPipe]) {
+      unsigned m[kPipe];
+      float du[kPipe], dv[kPipe], old[kPipe], cand[kPipe];
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) {
+        const int u = int(e[j].x), v = u + off;
+        m[j] = a.mask[u];
+        du[j] = __ldcg(d + u);
+        dv[j] = neighbour && unsigned(v) < a.n ? __ldcg(d + v) : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) {
+        const float x = __uint_as_float(e[j].y);
+        cand[j] = __fadd_rn(x, w);
+        const bool want = neighbour && ((m[j] >> lane) & 1u) && du[j] >= x && cand[j] < dv[j];
+        old[j] = want ? atomic_min_pos(d + int(e[j].x) + off, cand[j]) : -1.0f;
+      }
+      int n = 0;
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) n += __popc(__ballot_sync(kFull, old[j] > cand[j]));
+      if (!n) return;
+      const int slot = (r + 1) % 3;
+      int next = 0;
+      if (lane == 0) next = atomicAdd(&sh.qn[slot], n);
+      next = __shfl_sync(kFull, next, 0);
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) {
+        const int v = int(e[j].x) + off;
+        const int q = Places::take(next, old[j] > cand[j]);
+        if (!(old[j] > cand[j])) continue;
+        if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
+        else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
+      }
     };
-    // step A runs between barriers, with no relaxation in flight: the flag clear (a reduction,
-    // nothing to wait for) and the distance read need no order between them
-    int lo, hi;
-    if (own_share<C>(nc, kFloodStage, lo, hi)) {
-      unsigned long long *se = reinterpret_cast<unsigned long long *>(stage_bytes());
-      int *su = reinterpret_cast<int *>(se + kFloodStage);
-      for (int i = lo + int(threadIdx.x); i < hi; i += blockDim.x) {
-        const int u = __ldcg(cur + i);
-        atomicAnd(a.flags + u, ~kNearQueued);
-        const float du = __ldcg(d + u);
-        su[i - lo] = u;
-        se[i - lo] = (static_cast<unsigned long long>(__float_as_uint(du)) << 32) | a.mask[u];
+    for (int i = s.lo + warp * kPipe; i < s.hi; i += warps * kPipe) {
+      uint2 e[kPipe];
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) {
+        int q, at;
+        locate<C>(s, min(i + j, s.hi - 1), q, at);
+        e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue + at];
+        if (i + j >= s.hi) e[j].y = BK_INF_BITS;  // past the share: relaxes nothing
       }
-      G::sync();
-      for (int j = threadIdx.x; j < (hi - lo) * 26; j += blockDim.x) {
-        const int q = j / 26;
-        relax(se[q], su[q], j - 26 * q);
+      relax(e);
+    }
+    for (int i = (G::tid() >> 5) * kPipe; i < spilled; i += (G::threads() >> 5) * kPipe) {
+      uint2 e[kPipe];
+#pragma unroll
+      for (int j = 0; j < kPipe; ++j) {
+        const int u = __ldcg(cur + min(i + j, spilled - 1));
+        if (lane == 0 && i + j < spilled) atomicAnd(a.flags + u, ~spill_bit(r));
+        e[j] = make_uint2(unsigned(u), i + j < spilled ? __float_as_uint(__ldcg(d + u)) : BK_INF_BITS);
       }
-    } else {
-      for (int i = G::tid(); i < nc; i += G::threads()) {
-        const int u = __ldcg(cur + i);
-        atomicAnd(a.flags + u, ~kNearQueued);
-        const float du = __ldcg(d + u);
-        wide[i] = (static_cast<unsigned long long>(__float_as_uint(du)) << 32) | a.mask[u];
-      }
-      G::sync();
-      for (long long j = G::tid(); j < (long long)nc * 32; j += G::threads()) {
-        const int k = int(j & 31);
-        if (k >= 26) continue;
-        const int i = int(j >> 5);
-        relax(__ldcg(wide + i), __ldcg(cur + i), k);
-      }
+      relax(e);
     }
     G::sync();
   }
@@ -350,12 +505,11 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
   while (next_object<C>(a, sh, L, big)) {
     const int o = sh.obj;
     int *A = a.lists + sh.begin, *B = a.lists + a.F + sh.begin;
-    unsigned long long *wide = a.wide + sh.begin;
     int root = a.border_root[o];
     bool ok = true;
     if (root < 0) {
       // the farthest voxel (geometric distance) from the object's first voxel
-      ok = flood_geometric<C>(a, sh, L, a.daf, a.vox[sh.begin], A, B, wide);
+      ok = flood_geometric<C>(a, sh, L, a.daf, a.vox[sh.begin], A, B);
       if (ok) {
         const unsigned long long k = object_argmax<C>(a, sh, L, a.daf);
         root = int(0xFFFFFFFFu - unsigned(k));
@@ -363,7 +517,7 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
         G::sync();
       }
     }
-    if (ok) ok = flood_geometric<C>(a, sh, L, a.daf, root, A, B, wide, a.free_radius[o]);
+    if (ok) ok = flood_geometric<C>(a, sh, L, a.daf, root, A, B, a.free_radius[o]);
     if (!ok) {
       if (G::first()) a.status[o] = kBudget;
       G::sync();
@@ -397,7 +551,7 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
 // CTA takes small objects on its own: large objects start first (they set the kernel's length),
 // and no CTA idles while any object is left.
 template <int C>
-__global__ void __launch_bounds__(kEngineThreads, kEngineCtasPerSm) prepare_kernel(EngineArgs a) {
+__global__ void __launch_bounds__(kEngineThreads, 1) prepare_kernel(EngineArgs a) {
   prepare_loop<C>(a, true);
   prepare_loop<1>(a, false);
 }
@@ -409,167 +563,201 @@ __global__ void __launch_bounds__(kEngineThreads, kEngineCtasPerSm) prepare_kern
 // nearest rail as (distance bits << 32 | flat), BK_UNCLAIMED when no rail is reachable, and sets
 // L->status on a bound. The result is schedule-independent: every voxel at distance <= D (the
 // nearest rail's) is exact when the flood stops.
+// The far list holds the voxels first reached beyond T (at their first touch, so once each); one
+// whose distance is at most the T before has since been queued as near.
 template <int C>
 __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *L, int t, int *A, int *B, int *FA,
-                                       int *FB, int *touched, unsigned long long *wide) {
+                                       int *FB, int *touched) {
   using G = Group<C>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  uint2 *queue = reinterpret_cast<uint2 *>(queue_bytes());
+  const bool rails = a.fix_branching != 0;
   // without fix_branching there are no rails: a full SSSP from t (the parents' field)
+  const float ft = __ldcg(a.pdrf + t);
+  const bool on_rail = rails && ft == 0.0f;
   if (threadIdx.x == 0) {
     sh.rb = BK_UNCLAIMED;
-    sh.minfar = kMinFarNone;
+    sh.minfar[0] = kMinFarNone; sh.minfar[1] = kMinFarNone;
+    sh.qn[0] = 0; sh.qn[1] = 0; sh.qn[2] = 0;
+    sh.T = fmaxf(__fmul_rn(a.rail_band, ft), 1e-30f);
   }
   if (G::first()) {
     L->n_touch = 1;
     touched[0] = t;
-    L->cnt[0] = 0; L->cnt[1] = 0; L->cnt[2] = 0;
-    L->n_far = 0; L->n_keep = 0;
+    L->spilled[0] = 0; L->spilled[1] = 0; L->spilled[2] = 0;
+    L->far_n[0] = 0; L->far_n[1] = 0;
     a.dist[t] = 0.0f;
-    const float ft = __ldcg(a.pdrf + t);
-    if (a.fix_branching && ft == 0.0f) sh.rb = static_cast<unsigned long long>(unsigned(t));
-    else {
-      A[0] = t;
-      L->cnt[0] = 1;
-      atomicOr(a.flags + t, kNearQueued);
-      L->T = fmaxf(__fmul_rn(a.rail_band, ft), 1e-30f);
+    if (!on_rail) {
+      queue[0] = make_uint2(unsigned(t), 0u);
+      sh.qn[0] = 1;
     }
   }
   G::sync();
-  {
-    const unsigned long long rb = G::min_over(&sh.rb);
-    if (rb != BK_UNCLAIMED) {
-      G::sync();
-      return rb;
-    }
-  }
-  int *far = FA, *keep = FB;
+  if (on_rail) return static_cast<unsigned long long>(unsigned(t));
+  const bool neighbour = lane < 26;
+  const int off = neighbour ? sh.off[lane] : 0;
+  int p = 0;  // the far list in use
   const long long bound = capped(a, 16LL * sh.count + 256);
   long long work = 0;
   int r = 0;
-  for (;;) {
+  for (int band = 0;; ++band) {
+    int *far = p ? FB : FA, *keep = p ? FA : FB;
+    const float T = vload(&sh.T);
+    unsigned long long *minfar = &sh.minfar[band & 1];
+    // the nearest deferred voxel: the lanes' least (distance, penalty)
+    auto defer = [&](bool is, float dist, float penalty) {
+      const unsigned mine = is ? __float_as_uint(dist) : BK_INF_BITS;
+      const unsigned least = __reduce_min_sync(kFull, mine);
+      if (least < unsigned(vload(minfar) >> 32) && is && mine == least)
+        atomicMin(minfar, (static_cast<unsigned long long>(mine) << 32) | __float_as_uint(penalty));
+    };
     for (;; ++r) {
-      int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
-      const int nc = vload(&L->cnt[r % 3]);
-      if (nc == 0) break;
+      const Share s = share_of<C>(sh, r % 3, kFloodQueue);
+      const int spilled = vload(&L->spilled[r % 3]);
+      if (s.total + spilled == 0) break;
       if (++work > bound) {
         if (G::first()) L->status = kBudget;
         G::sync();
         return BK_UNCLAIMED;
       }
-      if (G::first()) { L->cnt[(r + 2) % 3] = 0; L->rounds += 1; }
-      const float T = vload(&L->T);
-      int *next_count = &L->cnt[(r + 1) % 3];
-      // step A: no relaxation is in flight between the barriers
-      auto stage = [&](int u) {
-        atomicAnd(a.flags + u, ~kNearQueued);
-        const float fu = a.pdrf[u];
-        const float du = __ldcg(a.dist + u);
-        const unsigned long long rb = vload(&sh.rb);
-        const float Tb = rb != BK_UNCLAIMED ? fminf(T, __uint_as_float(unsigned(rb >> 32))) : T;
-        const bool expand = (fu != 0.0f || !a.fix_branching) && du <= Tb;
-        return expand ? (static_cast<unsigned long long>(__float_as_uint(du)) << 32) | a.mask[u] : 0ull;
-      };
-      // step B, after the improvement of v to cand (from old)
-      auto improved = [&](int v, float cand, float fv, float old) {
-        {
-          if (old == inf()) touched[atomicAdd(&L->n_touch, 1)] = v;
-          if (a.fix_branching && fv == 0.0f)
-            atomicMin(&sh.rb, (static_cast<unsigned long long>(__float_as_uint(cand)) << 32) | unsigned(v));
-          const unsigned long long rb = vload(&sh.rb);
-          const float Tb = rb != BK_UNCLAIMED ? fminf(T, __uint_as_float(unsigned(rb >> 32))) : T;
-          if (cand <= Tb) {
-            if (!(atomicOr(a.flags + v, kNearQueued) & kNearQueued)) nxt[atomicAdd(next_count, 1)] = v;
-          } else {
-            atomicMin(&sh.minfar, (static_cast<unsigned long long>(__float_as_uint(cand)) << 32) | __float_as_uint(fv));
-            if (!(atomicOr(a.flags + v, kFarQueued) & kFarQueued)) far[atomicAdd(&L->n_far, 1)] = v;
+      if (threadIdx.x == 0) sh.qn[(r + 2) % 3] = 0;
+      if (G::first()) { L->spilled[(r + 2) % 3] = 0; L->rounds += 1; }
+      int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
+      auto relax = [&](const uint2 (&e)[kPipe]) {
+        unsigned m[kPipe];
+        float du[kPipe], dv[kPipe], fv[kPipe], old[kPipe], cand[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const int u = int(e[j].x), v = u + off;
+          m[j] = a.mask[u];
+          du[j] = __ldcg(a.dist + u);
+          const bool in = neighbour && unsigned(v) < a.n;
+          fv[j] = in ? a.pdrf[v] : 0.0f;
+          dv[j] = in ? __ldcg(a.dist + v) : 0.0f;
+        }
+        // beyond the nearest rail found so far nothing matters: its distance only falls
+        const float nearest = __uint_as_float(min(unsigned(vload(&sh.rb) >> 32), BK_INF_BITS));
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const float x = __uint_as_float(e[j].y);
+          cand[j] = vw_step(x, fv[j]);
+          const bool want = neighbour && ((m[j] >> lane) & 1u) && du[j] >= x && cand[j] < dv[j] && cand[j] <= nearest;
+          old[j] = want ? atomic_min_pos(a.dist + int(e[j].x) + off, cand[j]) : -1.0f;
+        }
+        bool near[kPipe], first[kPipe], beyond[kPipe], later[kPipe], any = false;
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const bool improved = old[j] > cand[j], rail = rails && fv[j] == 0.0f;
+          first[j] = improved && old[j] == inf();
+          near[j] = improved && !rail && cand[j] <= T;
+          beyond[j] = improved && !rail && cand[j] > T;
+          later[j] = beyond[j] && first[j];
+          any |= improved;
+          if (improved && rail)
+            atomicMin(&sh.rb, (static_cast<unsigned long long>(__float_as_uint(cand[j])) << 32) | unsigned(int(e[j].x) + off));
+        }
+        if (!__any_sync(kFull, any)) return;
+        const int slot = (r + 1) % 3;
+        Places at = reserve(near, first, later, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const int v = int(e[j].x) + off;
+          const int q = Places::take(at.queue, near[j]);
+          if (near[j]) {
+            if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
+            else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
           }
+          const int w = Places::take(at.touched, first[j]);
+          if (first[j]) touched[w] = v;
+          const int f = Places::take(at.far, later[j]);
+          if (later[j]) far[f] = v;
+          if (__any_sync(kFull, beyond[j])) defer(beyond[j], cand[j], fv[j]);
         }
       };
-      // step B: one (voxel, neighbour) item
-      auto relax = [&](unsigned long long e, int u, int k) {
-        if (!((unsigned(e) >> k) & 1u)) return;
-        const int v = u + sh.off[k];
-        const float fv = a.pdrf[v];
-        const float cand = vw_step(__uint_as_float(unsigned(e >> 32)), fv);
-        const float old = atomic_min_pos(a.dist + v, cand);
-        if (old > cand) improved(v, cand, fv, old);
-      };
-      int lo, hi;
-      if (own_share<C>(nc, kFloodStage, lo, hi)) {
-        unsigned long long *se = reinterpret_cast<unsigned long long *>(stage_bytes());
-        int *su = reinterpret_cast<int *>(se + kFloodStage);
-        for (int i = lo + int(threadIdx.x); i < hi; i += blockDim.x) {
-          const int u = __ldcg(cur + i);
-          su[i - lo] = u;
-          se[i - lo] = stage(u);
+      for (int i = s.lo + warp * kPipe; i < s.hi; i += warps * kPipe) {
+        uint2 e[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          int q, at;
+          locate<C>(s, min(i + j, s.hi - 1), q, at);
+          e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue + at];
+          if (i + j >= s.hi) e[j].y = BK_INF_BITS;  // past the share: relaxes nothing
         }
-        G::sync();
-        for (int j = threadIdx.x; j < (hi - lo) * 26; j += blockDim.x) {
-          const int q = j / 26;
-          relax(se[q], su[q], j - 26 * q);
+        relax(e);
+      }
+      for (int i = (G::tid() >> 5) * kPipe; i < spilled; i += (G::threads() >> 5) * kPipe) {
+        uint2 e[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const int u = __ldcg(cur + min(i + j, spilled - 1));
+          if (lane == 0 && i + j < spilled) atomicAnd(a.flags + u, ~spill_bit(r));
+          e[j] = make_uint2(unsigned(u), i + j < spilled ? __float_as_uint(__ldcg(a.dist + u)) : BK_INF_BITS);
         }
-      } else {
-        for (int i = G::tid(); i < nc; i += G::threads()) wide[i] = stage(__ldcg(cur + i));
-        G::sync();
-        for (long long j = G::tid(); j < (long long)nc * 32; j += G::threads()) {
-          const int k = int(j & 31);
-          if (k >= 26) continue;
-          const int i = int(j >> 5);
-          relax(__ldcg(wide + i), __ldcg(cur + i), k);
-        }
+        relax(e);
       }
       G::sync();
     }
-    // band end: the nearest rail is final once it lies inside the band
-    if (G::first()) {
-      L->flag = 0;
-      const unsigned long long rb = G::min_over(&sh.rb), minfar = G::min_over(&sh.minfar);
-      sh.rb = rb;
-      if (rb != BK_UNCLAIMED && __uint_as_float(unsigned(rb >> 32)) <= L->T) L->flag = 1;
-      else if (minfar == kMinFarNone) L->flag = 2;
-      else {
-        const float d = __uint_as_float(unsigned(minfar >> 32)), f = __uint_as_float(unsigned(minfar));
-        float w = __fmul_rn(a.rail_band, f);
-        const float lo = __fmul_rn(5e-4f, d);
-        if (!(w > lo)) w = lo;
-        L->T = __fadd_rn(d, w);
+    // Band end. Each CTA combines the group's copies by itself (they rest since the round's
+    // barrier; the next band's minima go to the other copy): the nearest rail is final once it lies
+    // inside the band or nothing deferred is as near.
+    if (warp == 0) {
+      unsigned long long rb = lane < C ? vload(of_rank<C>(&sh.rb, lane < C ? lane : 0)) : BK_UNCLAIMED;
+      unsigned long long mf = lane < C ? vload(of_rank<C>(minfar, lane < C ? lane : 0)) : kMinFarNone;
+#pragma unroll
+      for (int o = 1; o < C; o <<= 1) {
+        const unsigned long long x = __shfl_xor_sync(kFull, rb, o), y = __shfl_xor_sync(kFull, mf, o);
+        rb = x < rb ? x : rb;
+        mf = y < mf ? y : mf;
       }
-      L->n_keep = 0;
+      if (lane == 0) {
+        const float D = __uint_as_float(unsigned(rb >> 32)), d = __uint_as_float(unsigned(mf >> 32));
+        int flag = 0;
+        if (rb != BK_UNCLAIMED && (D <= T || mf == kMinFarNone || d > D)) flag = 1;
+        else if (mf == kMinFarNone) flag = 2;
+        else {
+          float w = __fmul_rn(a.rail_band, __uint_as_float(unsigned(mf)));
+          const float lo = __fmul_rn(5e-4f, d);
+          if (!(w > lo)) w = lo;
+          sh.T = __fadd_rn(d, w);
+        }
+        sh.flag = flag;
+        sh.rb = rb;
+        sh.minfar[(band + 1) & 1] = kMinFarNone;
+        sh.qn[(r + 2) % 3] = 0;
+      }
     }
-    G::sync();
-    // every CTA takes the combined rail and starts a fresh nearest-deferred minimum
-    if (threadIdx.x == 0) {
-      if (G::rank() != 0) sh.rb = vload(&L->rb);
-      sh.minfar = kMinFarNone;
-    }
+    if (G::first()) L->spilled[(r + 2) % 3] = 0;
     __syncthreads();
-    const int flag = vload(&L->flag);
+    const int flag = vload(&sh.flag);
     if (flag) {
       const unsigned long long rb = vload(&sh.rb);
       G::sync();
       return flag == 1 ? rb : BK_UNCLAIMED;
     }
-    // promote deferred voxels inside the new band into the current near list
-    int *cur = (r & 1) ? B : A;
-    const int nf = vload(&L->n_far);
-    const unsigned long long rb = vload(&sh.rb);
-    const float T = vload(&L->T);
-    const float Tp = rb != BK_UNCLAIMED ? fminf(T, __uint_as_float(unsigned(rb >> 32))) : T;
-    int *cur_count = &L->cnt[r % 3];
-    for (int i = G::tid(); i < nf; i += G::threads()) {
-      const int w = __ldcg(far + i);
-      const float dw = __ldcg(a.dist + w);
-      if (dw <= Tp) {
-        atomicAnd(a.flags + w, ~kFarQueued);
-        if (!(atomicOr(a.flags + w, kNearQueued) & kNearQueued)) cur[atomicAdd(cur_count, 1)] = w;
-      } else {
-        atomicMin(&sh.minfar, (static_cast<unsigned long long>(__float_as_uint(dw)) << 32) | __float_as_uint(a.pdrf[w]));
-        keep[atomicAdd(&L->n_keep, 1)] = w;
+    // the deferred voxels inside the new band become round r + 1's frontier (round r's counters may
+    // still be read by a CTA that finds them empty)
+    int *nxt = (r & 1) ? A : B;
+    const int nf = vload(&L->far_n[p]);
+    const float Tn = vload(&sh.T);
+    minfar = &sh.minfar[(band + 1) & 1];
+    for (int i0 = G::tid() - lane; i0 < nf; i0 += G::threads()) {
+      const int i = i0 + lane;
+      int w = 0;
+      float dw = 0.0f, fw = 0.0f;
+      if (i < nf) {
+        w = __ldcg(far + i);
+        dw = __ldcg(a.dist + w);
+        fw = a.pdrf[w];
       }
+      const bool waits = i < nf && dw > T;
+      queue_flood(a, sh, L, waits && dw <= Tn, w, __float_as_uint(dw), r, nxt);
+      append(waits && dw > Tn, w, keep, &L->far_n[p ^ 1]);
+      defer(waits && dw > Tn, dw, fw);
     }
     G::sync();
-    if (G::first()) L->n_far = L->n_keep;
-    int *tmp = far; far = keep; keep = tmp;
-    G::sync();
+    if (G::first()) L->far_n[p] = 0;
+    p ^= 1;
+    ++r;
   }
 }
 
@@ -579,6 +767,7 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
 // Writes the path target-first to out and returns its length (-1: no room).
 __device__ int backtrace(const EngineArgs &a, const Shared &sh, unsigned long long rb, int t, int *out, long long room) {
   const int lane = threadIdx.x & 31;
+  const int off = lane < 26 ? sh.off[lane] : 0;
   int cur = int(unsigned(rb));
   int len = 0;
   const long long bound = 2LL * sh.count + 2;
@@ -587,9 +776,11 @@ __device__ int backtrace(const EngineArgs &a, const Shared &sh, unsigned long lo
     if (cur != t) {
       const uint32_t m = a.mask[cur];
       unsigned db = BK_INF_BITS;
-      if (lane < 26 && ((m >> lane) & 1u)) {
-        const int u = cur + sh.off[lane];
-        if (a.pdrf[u] != 0.0f) db = __float_as_uint(__ldcg(a.dist + u));
+      const int u = cur + off;
+      if (lane < 26 && unsigned(u) < a.n) {  // read beside the mask, not after it
+        const float f = a.pdrf[u];
+        const unsigned du = __float_as_uint(__ldcg(a.dist + u));
+        if (((m >> lane) & 1u) && f != 0.0f) db = du;
       }
       const unsigned mb = __reduce_min_sync(kFull, db);
       if (mb < BK_INF_BITS) kb = int(__reduce_min_sync(kFull, db == mb ? unsigned(lane) : 64u));
@@ -718,235 +909,279 @@ __device__ __forceinline__ int band_of(unsigned mbits, float delta, int kmin) {
 // an alive neighbour v the source s when |aniso (v - s)| < scale DBF[s] + const, with
 // M' = max(M, |v - s|). Inside the band [k delta, (k+1) delta) offers claim at once, keeping the
 // least (M bits, source); rounds are synchronous (offers come from the keys of the round
-// boundary). Offers beyond the band wait; at the boundary each waiting voxel takes the best offer
-// of its claimed neighbours, the smallest names the next band, those inside it are claimed.
+// boundary). Offers beyond the band wait; at the boundary the best offer that each waiting voxel has
+// from its claimed neighbours counts: the smallest names the next band, those inside it are claimed.
 // Claimed voxels die. Returns false when a loop bound is hit.
+//
+// A waiting voxel's best offer is kept where offers are made (an atomic minimum on its key), not
+// gathered at the boundary: a voxel's key is final once its band has converged (every later offer
+// is at least the next band's), so an offer made from a voxel's final key stays right. A voxel whose
+// key improves again after its claim may have made offers from the earlier key: it is listed, and
+// at the boundary its waiting neighbours take their best offer from their claimed neighbours anew.
+// On the 512^3 dense workload 0.3 % of the claims are listed; gathering at every boundary instead
+// read 2.3 waiting voxels' neighbourhoods per foreground voxel and was 43 % of the trace's object time
+// (24 us a boundary).
+// A round has two steps with a group barrier between them. Step A takes the queued pairs whose key
+// is still the voxel's (the round boundary's keys) and stages per voxel what its offers share: mask,
+// key, position relative to the source and the source's reach. Step B makes the offers, a warp per
+// voxel: one L2 read per neighbour decides it (dead, holding a better key or offer, or out of reach:
+// done), an atomic follows only where the key changes.
 template <int C>
 __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int *path, int npath, int *A, int *B,
-                           int *FA, int *FB, int *touched, unsigned long long *wide, unsigned long long *side_u,
-                           unsigned long long *side_s) {
+                           int *FA, int *FB, int *touched, int *redo, unsigned long long *wide) {
   using G = Group<C>;
-  if (G::first()) { L->cnt[0] = 0; L->cnt[1] = 0; L->cnt[2] = 0; L->n_far = 0; L->n_keep = 0; L->n_touch = 0; }
-  G::sync();
-  for (int i = G::tid(); i < npath; i += G::threads()) {
-    const int p = __ldcg(path + i);
-    if (!__ldcg(a.alive + p)) continue;
-    const unsigned long long old = atomicMin(a.key + p, static_cast<unsigned long long>(unsigned(p)));
-    if (old == BK_UNCLAIMED) {
-      atomicOr(a.flags + p, kFront);
-      A[atomicAdd(&L->cnt[0], 1)] = p;
-      touched[atomicAdd(&L->n_touch, 1)] = p;
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  int4 *stage_id = reinterpret_cast<int4 *>(queue_bytes());           // voxel, mask, source + 1, M bits
+  float4 *stage_at = reinterpret_cast<float4 *>(stage_id + kInvalQueue);  // position - source's, reach
+  unsigned long long *queue_key = reinterpret_cast<unsigned long long *>(stage_at + kInvalQueue);
+  int *queue_vox = reinterpret_cast<int *>(queue_key + 2 * kInvalQueue);
+  if (threadIdx.x == 0) {
+    sh.qn[0] = 0; sh.qn[1] = 0; sh.qn[2] = 0;
+    sh.lowest[0] = BK_INF_BITS; sh.lowest[1] = BK_INF_BITS;
+  }
+  if (G::first()) {
+    L->spilled[0] = 0; L->spilled[1] = 0; L->spilled[2] = 0;
+    L->far_n[0] = 0; L->far_n[1] = 0;
+    L->n_touch = 0;
+    L->n_redo = 0;
   }
   G::sync();
-  int *far = FA, *keep = FB;
+  // queues the claimed voxels v (keys k) of the lanes with p in queue slot `slot`, buffer `buffer`
+  auto queue = [&](bool p, int v, unsigned long long k, int slot, int buffer, int *spill_list) {
+    const unsigned b = __ballot_sync(kFull, p);
+    if (!b) return;
+    const int at = queue_place(sh, p, b, slot);
+    if (!p) return;
+    if (at < kInvalQueue) {
+      queue_vox[buffer * kInvalQueue + at] = v;
+      queue_key[buffer * kInvalQueue + at] = k;
+    } else spill(a, v, kFront, spill_list, &L->spilled[slot]);
+  };
+  for (int i0 = G::tid() - lane; i0 < npath; i0 += G::threads()) {
+    const int i = i0 + lane;
+    const int v = i < npath ? __ldcg(path + i) : 0;
+    const unsigned long long k = unsigned(v) + 1u;
+    bool claimed = false;
+    if (i < npath && __ldcg(a.key + v) != 0) claimed = atomicMin(a.key + v, k) == BK_UNCLAIMED;
+    queue(claimed, v, k, 0, 0, A);
+    append(claimed, v, touched, &L->n_touch);
+  }
+  G::sync();
+  auto list_redo = [&](int v) {
+    const int at = atomicAdd(&L->n_redo, 1);
+    if (at < sh.count) redo[at] = v;
+  };
+  const bool neighbour = lane < 26;
+  const int off = neighbour ? sh.off[lane] : 0;
+  const float ox = neighbour ? float(c_dx[lane]) : 0.0f, oy = neighbour ? float(c_dy[lane]) : 0.0f,
+              oz = neighbour ? float(c_dz[lane]) : 0.0f;
+  int p = 0;  // the waiting list in use
   const long long bound = capped(a, 64LL * sh.count + 1024);
   long long work = 0;
   int band = 0, r = 0;
-  for (;;) {
+  for (int boundary = 0;; ++boundary) {
+    int *far = p ? FB : FA, *keep = p ? FA : FB;
     unsigned hi = __float_as_uint(__fmul_rn(float(band + 1), a.delta));
     for (;; ++r) {
-      int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
-      const int nc = vload(&L->cnt[r % 3]);
-      if (nc == 0) break;
+      const Share s = share_of<C>(sh, r % 3, kInvalQueue);
+      const int spilled = vload(&L->spilled[r % 3]);
+      if (s.total + spilled == 0) break;
       if (++work > bound) return false;
-      if (G::first()) { L->cnt[(r + 2) % 3] = 0; L->rounds += 1ull << 32; }
-      int *next_count = &L->cnt[(r + 1) % 3];
-      // step B: the offer of claimed u (key ku, positions (ux, uy, uz) and its source's, the
-      // source's reach) to its k-th neighbour; distance and reach checks come before the read of
-      // the neighbour's liveness (all three only filter)
-      auto offer = [&](int u, unsigned long long ku, int k, int ux, int uy, int uz, int qx, int qy, int qz, float rs) {
-        const float d = distance_to(a, ux + c_dx[k], uy + c_dy[k], uz + c_dz[k], qx, qy, qz);
-        if (d >= rs) return;
-        const int v = u + sh.off[k];
-        if (!a.alive[v]) return;
-        const int s = int(unsigned(ku));
-        unsigned mb = __float_as_uint(d);
-        const unsigned mu = unsigned(ku >> 32);
-        if (mb < mu) mb = mu;
-        if (mb < hi) {
-          const unsigned long long cand = (static_cast<unsigned long long>(mb) << 32) | unsigned(s);
-          const unsigned long long old = atomicMin(a.key + v, cand);
-          if (old > cand) {
-            if (old == BK_UNCLAIMED) touched[atomicAdd(&L->n_touch, 1)] = v;
-            if (!(atomicOr(a.flags + v, kFront) & kFront)) nxt[atomicAdd(next_count, 1)] = v;
+      if (threadIdx.x == 0) sh.qn[(r + 2) % 3] = 0;
+      if (G::first()) { L->spilled[(r + 2) % 3] = 0; L->rounds += 1ull << 32; }
+      int *cur = (r & 1) ? B : A, *nxt = (r & 1) ? A : B;
+      // step A: a thread per queued pair
+      for (int i0 = s.lo + warp * 32; i0 < s.hi; i0 += warps * 32) {
+        const int i = i0 + lane;
+        int q, at;
+        locate<C>(s, min(i, s.hi - 1), q, at);
+        if (i < s.hi) {
+          const int u = of_rank<C>(queue_vox, q)[(r & 1) * kInvalQueue + at];
+          const unsigned long long k = of_rank<C>(queue_key, q)[(r & 1) * kInvalQueue + at];
+          const int source = int(unsigned(k)) - 1;
+          const unsigned m = a.mask[u];
+          const bool current = __ldcg(a.key + u) == k;
+          const float rs = reach(a, source, sh.rscale, sh.rconst);
+          int x, y, z, qx, qy, qz;
+          coordinates(sh, u - sh.a0, x, y, z);
+          coordinates(sh, source - sh.a0, qx, qy, qz);
+          stage_id[i - s.lo] = make_int4(u, current ? int(m) : 0, source + 1, int(k >> 32));
+          stage_at[i - s.lo] = make_float4(float(x - qx), float(y - qy), float(z - qz), rs);
+        }
+      }
+      for (int i = G::tid(); i < spilled; i += G::threads()) {
+        const int u = __ldcg(cur + i);
+        wide[i] = __ldcg(a.key + u);
+        atomicAnd(a.flags + u, ~kFront);
+      }
+      G::sync();
+      // step B: a warp per voxel
+      auto offers = [&](const int4 (&e)[kPipe], const float4 (&at)[kPipe]) {
+        unsigned long long kv[kPipe], old[kPipe], cand[kPipe];
+        bool offer[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const bool is = neighbour && ((unsigned(e[j].y) >> lane) & 1u);
+          kv[j] = is ? __ldcg(a.key + e[j].x + off) : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const float dx = __fmul_rn(a.wx, at[j].x + ox), dy = __fmul_rn(a.wy, at[j].y + oy),
+                      dz = __fmul_rn(a.wz, at[j].z + oz);
+          const float d = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+          const unsigned mb = max(__float_as_uint(d), unsigned(e[j].w));
+          cand[j] = (static_cast<unsigned long long>(mb < hi ? mb : mb | 0x80000000u) << 32) | unsigned(e[j].z);
+          offer[j] = d < at[j].w && cand[j] < kv[j];
+          old[j] = 0;
+          if (offer[j]) old[j] = atomicMin(a.key + e[j].x + off, cand[j]);
+        }
+        bool claimed[kPipe], first[kPipe], waits[kPipe], any = false;
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          claimed[j] = old[j] > cand[j] && cand[j] < kWaits;
+          first[j] = claimed[j] && old[j] >= kWaits;
+          waits[j] = cand[j] >= kWaits && old[j] == BK_UNCLAIMED;
+          any |= claimed[j] || waits[j];
+          if (claimed[j] && !first[j]) list_redo(e[j].x + off);
+        }
+        if (!__any_sync(kFull, any)) return;
+        const int slot = (r + 1) % 3, buffer = ((r + 1) & 1) * kInvalQueue;
+        Places to = reserve(claimed, first, waits, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const int v = e[j].x + off;
+          const int q = Places::take(to.queue, claimed[j]);
+          if (claimed[j]) {
+            if (q < kInvalQueue) {
+              queue_vox[buffer + q] = v;
+              queue_key[buffer + q] = cand[j];
+            } else spill(a, v, kFront, nxt, &L->spilled[slot]);
           }
-        } else if (__ldcg(a.key + v) == BK_UNCLAIMED) {
-          if (!(atomicOr(a.flags + v, kWaiting) & kWaiting)) far[atomicAdd(&L->n_far, 1)] = v;
+          const int w = Places::take(to.touched, first[j]);
+          if (first[j]) touched[w] = v;
+          const int f = Places::take(to.far, waits[j]);
+          if (waits[j]) far[f] = v;
         }
       };
-      int lo, hi_i;
-      if (own_share<C>(nc, kInvalStage, lo, hi_i)) {
-        // step A: the round boundary's key of each frontier voxel, its mask, both positions and
-        // the source's reach, in this CTA's shared memory
-        unsigned long long *skey = reinterpret_cast<unsigned long long *>(stage_bytes());
-        unsigned long long *spu = skey + kInvalStage, *sps = spu + kInvalStage;
-        int *su = reinterpret_cast<int *>(sps + kInvalStage);
-        unsigned *smask = reinterpret_cast<unsigned *>(su + kInvalStage);
-        float *sreach = reinterpret_cast<float *>(smask + kInvalStage);
-        for (int i = lo + int(threadIdx.x); i < hi_i; i += blockDim.x) {
-          const int u = __ldcg(cur + i);
-          const unsigned long long k = __ldcg(a.key + u);
-          atomicAnd(a.flags + u, ~kFront);
-          const int q = i - lo;
-          su[q] = u;
-          skey[q] = k;
-          smask[q] = a.mask[u];
-          sreach[q] = reach(a, int(unsigned(k)), sh.rscale, sh.rconst);
-          int x, y, z;
-          unravel3(u - sh.a0, sh.sx, sh.sy, x, y, z);
-          spu[q] = pack3(x, y, z);
-          unravel3(int(unsigned(k)) - sh.a0, sh.sx, sh.sy, x, y, z);
-          sps[q] = pack3(x, y, z);
+      const int staged = s.hi - s.lo;
+      for (int i = warp * kPipe; i < staged; i += warps * kPipe) {
+        int4 e[kPipe];
+        float4 at[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          e[j] = stage_id[min(i + j, staged - 1)];
+          at[j] = stage_at[min(i + j, staged - 1)];
+          if (i + j >= staged) e[j].y = 0;
         }
-        G::sync();
-        for (int j = threadIdx.x; j < (hi_i - lo) * 26; j += blockDim.x) {
-          const int q = j / 26, k = j - 26 * q;
-          if (!((smask[q] >> k) & 1u)) continue;
-          int ux, uy, uz, qx, qy, qz;
-          unpack3(spu[q], ux, uy, uz);
-          unpack3(sps[q], qx, qy, qz);
-          offer(su[q], skey[q], k, ux, uy, uz, qx, qy, qz, sreach[q]);
+        offers(e, at);
+      }
+      for (int i = (G::tid() >> 5) * kPipe; i < spilled; i += (G::threads() >> 5) * kPipe) {
+        int4 e[kPipe];
+        float4 at[kPipe];
+#pragma unroll
+        for (int j = 0; j < kPipe; ++j) {
+          const int w = min(i + j, spilled - 1), u = __ldcg(cur + w);
+          const unsigned long long k = __ldcg(wide + w);
+          const int source = int(unsigned(k)) - 1;
+          int x, y, z, qx, qy, qz;
+          coordinates(sh, u - sh.a0, x, y, z);
+          coordinates(sh, source - sh.a0, qx, qy, qz);
+          e[j] = make_int4(u, i + j < spilled ? int(a.mask[u]) : 0, source + 1, int(k >> 32));
+          at[j] = make_float4(float(x - qx), float(y - qy), float(z - qz), reach(a, source, sh.rscale, sh.rconst));
         }
-      } else {
-        // step A: the round boundary's key of each frontier voxel, and both positions
-        for (int i = G::tid(); i < nc; i += G::threads()) {
-          const int u = __ldcg(cur + i);
-          const unsigned long long k = __ldcg(a.key + u);
-          atomicAnd(a.flags + u, ~kFront);
-          wide[i] = k;
-          int x, y, z;
-          unravel3(u - sh.a0, sh.sx, sh.sy, x, y, z);
-          side_u[i] = pack3(x, y, z);
-          unravel3(int(unsigned(k)) - sh.a0, sh.sx, sh.sy, x, y, z);
-          side_s[i] = pack3(x, y, z);
-        }
-        G::sync();
-        for (long long j = G::tid(); j < (long long)nc * 32; j += G::threads()) {
-          const int k = int(j & 31);
-          if (k >= 26) continue;
-          const int i = int(j >> 5);
-          const int u = __ldcg(cur + i);
-          if (!((a.mask[u] >> k) & 1u)) continue;
-          const unsigned long long ku = __ldcg(wide + i);
-          int ux, uy, uz, qx, qy, qz;
-          unpack3(__ldcg(side_u + i), ux, uy, uz);
-          unpack3(__ldcg(side_s + i), qx, qy, qz);
-          offer(u, ku, k, ux, uy, uz, qx, qy, qz, reach(a, int(unsigned(ku)), sh.rscale, sh.rconst));
-        }
+        offers(e, at);
       }
       G::sync();
     }
-    const int nf = vload(&L->n_far);
+    const int nf = vload(&L->far_n[p]);
     if (nf == 0) break;
     if (++work > bound) return false;
-    // band boundary: every waiting voxel pulls the best offer of its claimed neighbours
-    if (threadIdx.x == 0) sh.lowest = BK_INF_BITS;
-    if (G::first()) L->n_keep = 0;
-    // the offer of claimed neighbour key ku to waiting voxel c at (x, y, z), or ~0
-    auto pull = [&](unsigned long long ku, int x, int y, int z) -> unsigned long long {
-      const int s = int(unsigned(ku));
-      int qx, qy, qz;
-      unravel3(s - sh.a0, sh.sx, sh.sy, qx, qy, qz);
-      const float d = distance_to(a, x, y, z, qx, qy, qz);
-      if (d >= reach(a, s, sh.rscale, sh.rconst)) return ~0ull;
-      unsigned mb = __float_as_uint(d);
-      const unsigned mu = unsigned(ku >> 32);
-      if (mb < mu) mb = mu;
-      atomicMin(&sh.lowest, mb);
-      return (static_cast<unsigned long long>(mb) << 32) | unsigned(s);
-    };
-    // claim the waiting voxel c with best offer b inside the new band, or keep it waiting
-    auto settle = [&](int c, unsigned long long b, int *cur, int *cur_count) {
-      if (b == kClaimedMark) return;
-      if (b == BK_UNCLAIMED) { atomicAnd(a.flags + c, ~kWaiting); return; }
-      if (unsigned(b >> 32) < hi) {
-        a.key[c] = b;
-        touched[atomicAdd(&L->n_touch, 1)] = c;
-        atomicAnd(a.flags + c, ~kWaiting);
-        atomicOr(a.flags + c, kFront);
-        cur[atomicAdd(cur_count, 1)] = c;
-      } else {
-        keep[atomicAdd(&L->n_keep, 1)] = c;
-      }
-    };
-    int lo, hi_f;
-    if (own_share<C>(nf, kBandStage, lo, hi_f)) {
-      // this CTA's waiting voxels in shared memory: nothing writes a key before the claims, which
-      // come after a group barrier, so the pulls only wait for this CTA's staging
-      unsigned long long *sbest = reinterpret_cast<unsigned long long *>(stage_bytes());
-      unsigned long long *spc = sbest + kBandStage;
-      int *sc = reinterpret_cast<int *>(spc + kBandStage);
-      unsigned *smask = reinterpret_cast<unsigned *>(sc + kBandStage);
-      for (int i = lo + int(threadIdx.x); i < hi_f; i += blockDim.x) {
-        const int c = __ldcg(far + i);
-        const int q = i - lo;
-        sc[q] = c;
-        sbest[q] = __ldcg(a.key + c) != BK_UNCLAIMED ? kClaimedMark : BK_UNCLAIMED;
-        smask[q] = a.mask[c];
-        int x, y, z;
-        unravel3(c - sh.a0, sh.sx, sh.sy, x, y, z);
-        spc[q] = pack3(x, y, z);
-      }
-      __syncthreads();
-      for (int j = threadIdx.x; j < (hi_f - lo) * 26; j += blockDim.x) {
-        const int q = j / 26, k = j - 26 * q;
-        if (sbest[q] == kClaimedMark || !((smask[q] >> k) & 1u)) continue;
-        const unsigned long long ku = __ldcg(a.key + sc[q] + sh.off[k]);
-        if (ku == BK_UNCLAIMED) continue;
-        int x, y, z;
-        unpack3(spc[q], x, y, z);
-        const unsigned long long o = pull(ku, x, y, z);
-        if (o != ~0ull) atomicMin(sbest + q, o);
+    // band boundary: the neighbours of the listed voxels first, a warp per listed voxel and then per
+    // waiting neighbour of it (the neighbours' keys, then their sources' reach)
+    const int nr = vload(&L->n_redo);
+    if (nr > 0) {
+      const bool all = nr > sh.count;  // more than the list holds: every waiting voxel
+      const int m = all ? nf : nr;
+      for (int i = G::tid() >> 5; i < m; i += G::threads() >> 5) {
+        const int u = __ldcg((all ? far : redo) + i);
+        unsigned again = 0;
+        if (!all) {
+          const unsigned long long kc = neighbour && ((a.mask[u] >> lane) & 1u) ? __ldcg(a.key + u + off) : 0ull;
+          again = __ballot_sync(kFull, kc >= kWaits && kc != BK_UNCLAIMED);
+        } else again = __ldcg(a.key + u) >= kWaits ? 1u << 26 : 0u;
+        for (; again; again &= again - 1) {
+          const int k = __ffs(again) - 1;
+          const int c = all ? u : u + sh.off[k];
+          unsigned long long ku = neighbour && ((a.mask[c] >> lane) & 1u) ? __ldcg(a.key + c + off) : 0ull;
+          if (ku >= kWaits) ku = 0;
+          unsigned mb = ~0u, from = ~0u;
+          if (ku) {
+            const int source = int(unsigned(ku)) - 1;
+            int x, y, z, qx, qy, qz;
+            coordinates(sh, c - sh.a0, x, y, z);
+            coordinates(sh, source - sh.a0, qx, qy, qz);
+            const float d = distance_to(a, x, y, z, qx, qy, qz);
+            if (d < reach(a, source, sh.rscale, sh.rconst)) {
+              mb = max(__float_as_uint(d), unsigned(ku >> 32)) | 0x80000000u;
+              from = unsigned(ku);
+            }
+          }
+          const unsigned least = __reduce_min_sync(kFull, mb);
+          from = __reduce_min_sync(kFull, mb == least ? from : ~0u);
+          // no offer left: all ones, and the voxel leaves the list below
+          if (lane == 0) a.key[c] = (static_cast<unsigned long long>(least) << 32) | from;
+        }
       }
       G::sync();
-      const unsigned lowest = G::min_over(&sh.lowest);
-      if (lowest != BK_INF_BITS) band = band_of(lowest, a.delta, band + 1);
-      hi = __float_as_uint(__fmul_rn(float(band + 1), a.delta));
-      int *cur = (r & 1) ? B : A;
-      for (int i = lo + int(threadIdx.x); i < hi_f; i += blockDim.x) settle(sc[i - lo], sbest[i - lo], cur, &L->cnt[r % 3]);
-    } else {
-      for (int i = G::tid(); i < nf; i += G::threads()) {
-        const int c = __ldcg(far + i);
-        wide[i] = __ldcg(a.key + c) != BK_UNCLAIMED ? kClaimedMark : BK_UNCLAIMED;
-        int x, y, z;
-        unravel3(c - sh.a0, sh.sx, sh.sy, x, y, z);
-        side_u[i] = pack3(x, y, z);
+      if (G::first()) L->n_redo = 0;
+    }
+    // the smallest offer names the next band. The first strip's voxels stay in registers.
+    unsigned lowest = BK_INF_BITS;
+    int c0 = 0;
+    unsigned long long k0 = 0;
+    for (int i0 = G::tid() - lane; i0 < nf; i0 += G::threads()) {
+      const int i = i0 + lane;
+      int c = 0;
+      unsigned long long k = 0;
+      if (i < nf) {
+        c = __ldcg(far + i);
+        k = __ldcg(a.key + c);
       }
-      G::sync();
-      for (long long j = G::tid(); j < (long long)nf * 32; j += G::threads()) {
-        const int k = int(j & 31);
-        if (k >= 26) continue;
-        const int i = int(j >> 5);
-        if (__ldcg(wide + i) == kClaimedMark) continue;
-        const int c = __ldcg(far + i);
-        if (!((a.mask[c] >> k) & 1u)) continue;
-        const unsigned long long ku = __ldcg(a.key + c + sh.off[k]);
-        if (ku == BK_UNCLAIMED) continue;
-        int x, y, z;
-        unpack3(__ldcg(side_u + i), x, y, z);
-        const unsigned long long o = pull(ku, x, y, z);
-        if (o != ~0ull) atomicMin(wide + i, o);
+      if (k >= kWaits && k != BK_UNCLAIMED) lowest = min(lowest, unsigned(k >> 32) & 0x7FFFFFFFu);
+      if (i < G::threads()) { c0 = c; k0 = k; }
+    }
+    lowest = __reduce_min_sync(kFull, lowest);
+    if (lane == 0 && lowest != BK_INF_BITS) atomicMin(&sh.lowest[boundary & 1], lowest);
+    G::sync();
+    lowest = __reduce_min_sync(kFull, lane < C ? vload(of_rank<C>(&sh.lowest[boundary & 1], lane < C ? lane : 0)) : BK_INF_BITS);
+    if (threadIdx.x == 0) sh.lowest[(boundary + 1) & 1] = BK_INF_BITS;
+    if (lowest != BK_INF_BITS) band = band_of(lowest, a.delta, band + 1);
+    hi = __float_as_uint(__fmul_rn(float(band + 1), a.delta));
+    // offers inside it claim, the rest wait on
+    int *cur = (r & 1) ? B : A;
+    for (int i0 = G::tid() - lane; i0 < nf; i0 += G::threads()) {
+      const int i = i0 + lane;
+      int c = c0;
+      unsigned long long k = k0;
+      if (i >= G::threads()) {
+        c = i < nf ? __ldcg(far + i) : 0;
+        k = i < nf ? __ldcg(a.key + c) : 0;
       }
-      G::sync();
-      const unsigned lowest = G::min_over(&sh.lowest);
-      if (lowest != BK_INF_BITS) band = band_of(lowest, a.delta, band + 1);
-      hi = __float_as_uint(__fmul_rn(float(band + 1), a.delta));
-      int *cur = (r & 1) ? B : A;
-      for (int i = G::tid(); i < nf; i += G::threads()) settle(__ldcg(far + i), __ldcg(wide + i), cur, &L->cnt[r % 3]);
+      const bool waits = k >= kWaits && k != BK_UNCLAIMED;
+      k &= ~kWaits;
+      const bool claims = waits && unsigned(k >> 32) < hi;
+      if (claims) a.key[c] = k;
+      queue(claims, c, k, r % 3, r & 1, cur);
+      append(claims, c, touched, &L->n_touch);
+      append(waits && !claims, c, keep, &L->far_n[p ^ 1]);
     }
     G::sync();
-    if (G::first()) L->n_far = L->n_keep;
-    int *tmp = far; far = keep; keep = tmp;
-    G::sync();
+    if (G::first()) L->far_n[p] = 0;
+    p ^= 1;
   }
+  // the claimed voxels die
   const int nt = vload(&L->n_touch);
-  for (int i = G::tid(); i < nt; i += G::threads()) {
-    const int v = __ldcg(touched + i);
-    a.alive[v] = 0;
-    a.key[v] = BK_UNCLAIMED;
-    atomicAnd(a.flags + v, ~(kFront | kWaiting));
-  }
+  for (int i = G::tid(); i < nt; i += G::threads()) a.key[__ldcg(touched + i)] = 0;
   G::sync();
   return true;
 }
@@ -965,8 +1200,8 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
       G::sync();
       continue;
     }
-    int *L0 = a.lists + sh.begin, *L1 = L0 + a.F, *L2 = L1 + a.F, *L3 = L2 + a.F, *L4 = L3 + a.F;
-    unsigned long long *wide = a.wide + sh.begin, *side_u = a.side + sh.begin, *side_s = a.side + a.F + sh.begin;
+    int *L0 = a.lists + sh.begin, *L1 = L0 + a.F, *L2 = L1 + a.F, *L3 = L2 + a.F, *L4 = L3 + a.F, *L5 = L4 + a.F;
+    unsigned long long *wide = a.wide + sh.begin;
     int *store = a.store + a.store_begin[o];
     const long long store_cap = a.store_cap[o];
     int *rec_start = a.rec_start + a.rec_begin[o], *rec_len = a.rec_len + a.rec_begin[o];
@@ -1018,7 +1253,7 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
             if (threadIdx.x == 0) sh.pos = INT32_MAX;
             G::sync();
             const int pos = cursor + G::tid();
-            if (pos < sh.count && __ldcg(a.alive + order[pos])) atomicMin(&sh.pos, unsigned(pos));
+            if (pos < sh.count && __ldcg(a.key + order[pos]) != 0) atomicMin(&sh.pos, unsigned(pos));
             G::sync();
             const int found = int(G::min_over(&sh.pos));
             G::sync();
@@ -1035,12 +1270,11 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
         if (G::first()) store[used] = sh.root;  // the ball's one source (the slot is reused)
         G::sync();
       } else if (step == 1 || a.fix_branching) {
-        const unsigned long long rb = railroad<C>(a, sh, L, step == 1 ? sh.root : t, L0, L1, L2, L3, L4, wide);
+        const unsigned long long rb = railroad<C>(a, sh, L, step == 1 ? sh.root : t, L0, L1, L2, L3, L4);
         lap(1);
         if (vload(&L->status) != kOk) { status = vload(&L->status); break; }
         const int nt = vload(&L->n_touch);
-        if (step == 1) {  // the parents' field stays; its queue flags are cleared now
-          for (int i = G::tid(); i < nt; i += G::threads()) atomicAnd(a.flags + __ldcg(L4 + i), ~(kNearQueued | kFarQueued));
+        if (step == 1) {  // the parents' field stays
           if (G::first()) { s_work[0] += nt; s_work[1] += nt; }
           if (threadIdx.x == 0) sh.step = 2;  // every CTA of the group moves on (each has its own copy)
           G::sync();
@@ -1051,11 +1285,7 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
           // stage painted without refreshing the field). A target of the DAF order would be picked
           // again and again, so the object ends here (trace.cu:218-224); a manual target leaves an
           // empty path. Either way the flood's state goes back to rest first.
-          for (int i = G::tid(); i < nt; i += G::threads()) {
-            const int v = __ldcg(L4 + i);
-            a.dist[v] = inf();
-            atomicAnd(a.flags + v, ~(kNearQueued | kFarQueued));
-          }
+          for (int i = G::tid(); i < nt; i += G::threads()) a.dist[__ldcg(L4 + i)] = inf();
           if (G::first()) s_work[1] += nt;
           if (threadIdx.x == 0 && !ordered) sh.skipped += 1;  // every CTA keeps its own copy
           G::sync();
@@ -1074,7 +1304,6 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
           const int v = __ldcg(L4 + i);
           settled += __ldcg(a.dist + v) <= D;
           a.dist[v] = inf();
-          atomicAnd(a.flags + v, ~(kNearQueued | kFarQueued));
         }
         settled = __reduce_add_sync(kFull, settled);
         if ((threadIdx.x & 31) == 0) atomicAdd(&s_work[0], (unsigned long long)settled);
@@ -1109,7 +1338,7 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
         sh.rconst = ball ? a.soma_constant : a.constant;
       }
       __syncthreads();
-      if (!invalidate<C>(a, sh, L, store + used, len, L0, L1, L2, L3, L4, wide, side_u, side_s)) {
+      if (!invalidate<C>(a, sh, L, store + used, len, L0, L1, L2, L3, L4, L5, wide)) {
         status = kBudget;
         break;
       }
@@ -1153,7 +1382,7 @@ template <int C>
 // The first a.lone_first clusters start on the small objects (each CTA alone, largest first) and
 // then join the large ones; the others take the large objects first. So the longest lone-CTA
 // objects run beside the clusters' objects from the start instead of after them.
-__global__ void __launch_bounds__(kEngineThreads, kEngineCtasPerSm) trace_kernel(EngineArgs a) {
+__global__ void __launch_bounds__(kEngineThreads, 1) trace_kernel(EngineArgs a) {
   if (int(blockIdx.x) / C < a.lone_first) {
     trace_loop<1>(a, false);
     trace_loop<C>(a, true);
@@ -1211,24 +1440,29 @@ void launch(const void *kernel, int ctas, const EngineArgs &a, int nbig, cudaStr
 
 }  // namespace
 
-long long trace_cluster_voxels(long long foreground) {
+// The engine's resident CTAs on the current device.
+static long long resident_ctas() {
   static std::mutex lock;
-  static std::map<int, long long> known;  // resident engine CTAs per device
+  static std::map<int, long long> known;
   int device = 0;
   BK_CUDA(cudaGetDevice(&device));
-  long long ctas = 0;
-  {
-    std::lock_guard<std::mutex> guard(lock);
-    auto it = known.find(device);
-    if (it == known.end()) {
-      int sms = 1, per_sm = 1;
-      BK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-      BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas>, kEngineThreads, 0));
-      it = known.emplace(device, std::max(1LL, (long long)sms * per_sm)).first;
-    }
-    ctas = it->second;
+  std::lock_guard<std::mutex> guard(lock);
+  auto it = known.find(device);
+  if (it == known.end()) {
+    int sms = 1, per_sm = 1;
+    BK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas>, kEngineThreads, 0));
+    it = known.emplace(device, std::max(1LL, (long long)sms * per_sm)).first;
   }
-  return std::max(kTraceClusterFloor, foreground / (2 * ctas));
+  return it->second;
+}
+
+long long trace_cluster_voxels(long long foreground) {
+  return std::max(kTraceClusterFloor, foreground / resident_ctas());
+}
+
+long long prepare_cluster_voxels(long long foreground) {
+  return std::max(kPrepareClusterFloor, foreground / (2 * resident_ctas()));
 }
 
 int cluster_ctas(long long largest, long long foreground) {

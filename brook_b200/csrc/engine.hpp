@@ -11,13 +11,16 @@
 
 namespace bk {
 
-constexpr int kEngineThreads = 512;  // threads per CTA
+// Threads per CTA: one CTA per SM at the 64 registers its floods need without spills. A frontier
+// voxel is a warp's work, so an object's rounds are as fast as its warps are many, and a lone CTA's
+// barrier costs a fraction of a cluster's. On the 512^3 dense workload (trace ms, every object on one
+// CTA) 256 threads 57.7, 512 35.7, 1024 29.7.
+constexpr int kEngineThreads = 1024;
 
 // Per-voxel flag bits (uint32 per voxel, 0 at rest).
-constexpr unsigned kNearQueued = 1u;   // railroad / flood: in the next near list
-constexpr unsigned kFarQueued = 2u;    // railroad: on the far list
-constexpr unsigned kFront = 4u;        // invalidation: in the next frontier
-constexpr unsigned kWaiting = 8u;      // invalidation: on the waiting list
+constexpr unsigned kSpillEven = 1u;    // floods: on the spill list of an even round
+constexpr unsigned kSpillOdd = 2u;     // floods: on the spill list of an odd round
+constexpr unsigned kFront = 4u;        // invalidation: on the next round's spill list
 constexpr unsigned kOnPath = 16u;      // without fix_branching: on a stored path of the object
 
 enum EngineStatus : int {
@@ -40,8 +43,8 @@ struct EngineArgs {
   float *dist;           // railroad distances, +inf at rest
   float *daf;            // DAF, +inf before prepare
   uint32_t *flags;       // 0 at rest
-  uint8_t *alive;
-  unsigned long long *key;  // invalidation keys, all ones at rest
+  unsigned long long *key;  // invalidation keys: all ones for a living voxel at rest, 0 for a dead one
+  unsigned n;               // voxels of the flat space
 
   int nobj;
   const int *obj_begin;  // offset of the object's voxels in vox and in the list pool
@@ -52,9 +55,8 @@ struct EngineArgs {
   int lone_first;        // trace: clusters [0, lone_first) take the small objects first
   int *queue;            // two work counters (large, small), both 0 at launch
   int *status;           // per object
-  int *lists;            // 5 lists of F ints: list w of object o at lists + w * F + obj_begin[o]
-  unsigned long long *wide;  // F entries: object o at wide + obj_begin[o] (per-entry staging)
-  unsigned long long *side;  // 2F entries: two more staging arrays (packed coordinates)
+  int *lists;            // 6 lists of F ints: list w of object o at lists + w * F + obj_begin[o]
+  unsigned long long *wide;  // F entries: object o at wide + obj_begin[o] (a spilled frontier's keys)
   long long F;
 
   // prepare
@@ -107,23 +109,29 @@ struct EngineArgs {
   int grid_percent;
 };
 
-// Objects with at least kPrepareClusterVoxels voxels (preparation) or more voxels than
-// trace_cluster_voxels (tracing) run on a cluster of CTAs that share the object's frontiers
-// through distributed shared memory; smaller objects on one CTA each. Tracing keeps clusters for
-// the objects whose lone-CTA chain would outlast the kernel's even share of the work: a cluster
-// spends more CTA-time per object than a lone CTA, which pays only where the object's own chain
-// would otherwise set the kernel's length. Clusters have kClusterCtas CTAs, or kWideClusterCtas
-// when the largest object holds at least 1/kWideClusterShare of the foreground (its chain is
-// then the kernel's length whatever else runs beside it).
+// Objects with at least prepare_cluster_voxels voxels (preparation) or trace_cluster_voxels (tracing)
+// run on a cluster of CTAs that share the object's frontiers through distributed shared memory;
+// smaller objects on one CTA each. A cluster's round pays for its barrier and for remote counters and
+// queues, so it spends more CTA-time on an object than a lone CTA, which pays only where the
+// object's own chain would outlast an even share of the work over all CTAs. Clusters have
+// kClusterCtas CTAs, or kWideClusterCtas when the largest object holds at least 1/kWideClusterShare of
+// the foreground (its chain is then the kernel's length whatever else runs beside it).
 constexpr int kClusterCtas = 4;
 constexpr int kWideClusterCtas = 8;
 constexpr long long kWideClusterShare = 16;
 int cluster_ctas(long long largest, long long foreground);
-constexpr int kPrepareClusterVoxels = 8192;
-constexpr long long kTraceClusterFloor = 16384;
-// Half the foreground voxels per resident engine CTA (largest-first scheduling then leaves the
-// clusters' objects as the only ones longer than a CTA's share), at least kTraceClusterFloor.
+// Tracing: the foreground voxels per resident CTA, at least kTraceClusterFloor. Measured (trace ms with
+// clusters from 2048, 16384 and 65536 voxels, and without): 512^3 dense (share 190 k) 79.0, 71.7,
+// 43.1, 29.7; 16 volumes in a batch (56 k) 33.5, 24.9, 10.0, 9.7; 256^3 dense (24 k) 11.8, 11.7, 11.6,
+// 17.8; 128^3 tubes (3 k; objects up to 61 k) 7.9, 7.8, 9.1, 9.1; a 48^3 request (objects of 16-31 k)
+// 4.9, 4.9, 4.1, 4.1.
+constexpr long long kTraceClusterFloor = 32768;
 long long trace_cluster_voxels(long long foreground);
+// Preparation, whose floods have frontiers ten times as wide: half that share, at least
+// kPrepareClusterFloor (prepare ms, the same columns: 20.9, 18.3, 14.4, 12.9; 6.4, 4.8, 3.9, 4.1; 2.6, 2.9,
+// 5.1, 6.2; 1.2, 1.1, 2.6, 2.5; 0.48, 0.61, 1.1, 1.1).
+constexpr long long kPrepareClusterFloor = 4096;
+long long prepare_cluster_voxels(long long foreground);
 
 // One pass of the engine: clusters take schedule[0, nbig) (large objects, largest first), then
 // every CTA takes schedule[nbig, nobj) alone. queue[0] and queue[1] must be zero.

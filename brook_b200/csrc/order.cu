@@ -47,11 +47,6 @@ __global__ void arena_object_keys(const int *vox, ArenaObject at, uint32_t *keys
   if (i < n) keys[i] = uint32_t(at(vox[i]));
 }
 
-__global__ void mark_alive(const int *vox, uint8_t *alive, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) alive[vox[i]] = 1;
-}
-
 // The composite key's fields for list position i of object o: o << (lbits + 31) | (0x7FFFFFFF -
 // daf bits) << lbits | (2^lbits - 1 - position in o).
 struct WideKey {
@@ -130,7 +125,7 @@ __global__ void unpack_order96(const WideKey *keys, const int *vox, const int *b
 }  // namespace
 
 Buffer<int> arena_object_voxels(Context &ctx, const uint32_t *ids, long long n, const std::vector<ArenaVolume> &volumes,
-                                const std::vector<int> &object_of, int nobj, long long total, uint8_t *alive) {
+                                const std::vector<int> &object_of, int nobj, long long total) {
   cudaStream_t s = ctx.stream();
   Buffer<int> vox(ctx, total > 0 ? total : 1);
   if (total == 0 || volumes.empty()) {
@@ -172,8 +167,6 @@ Buffer<int> arena_object_voxels(Context &ctx, const uint32_t *ids, long long n, 
   scratch = Buffer<unsigned char>(ctx, temp);
   BK_CUDA(cub::DeviceRadixSort::SortPairs(scratch.data(), temp, keys.data(), keys_out.data(), picked.data(), vox.data(),
                                           (int)total, 0, bits, s));
-  mark_alive<<<blocks_for(total), 256, 0, s>>>(vox.data(), alive, (int)total); ++ctx.launches;
-  BK_CUDA(cudaGetLastError());
   if (count.download(1)[0] != total) throw std::runtime_error("object voxel count mismatch");
   return vox;
 }

@@ -11,10 +11,10 @@ struct ArenaVolume {
   int id_base;
 };
 // Voxels of every object over all volumes of the arena in one selection and one sort: grouped by
-// global object index (object_of[id_base + id] >= 0), ascending in arena flat index. The picked
-// voxels are also marked in `alive` (zeroed by the caller). `total` is the objects' voxel count.
+// global object index (object_of[id_base + id] >= 0), ascending in arena flat index. `total` is the
+// objects' voxel count.
 Buffer<int> arena_object_voxels(Context &ctx, const uint32_t *ids, long long n, const std::vector<ArenaVolume> &volumes,
-                                const std::vector<int> &object_of, int nobj, long long total, uint8_t *alive);
+                                const std::vector<int> &object_of, int nobj, long long total);
 // Per object (voxels [begin[o], begin[o+1]) of the list, the last to `total`): its voxels by
 // descending DAF (inf -> 0), ties -> higher flat first. `largest` is the largest object's voxel
 // count; `wide` forces the (32, 64)-bit key even where 64 bits would hold it.

@@ -533,15 +533,13 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   // global per-voxel state
   Buffer<float> pdrf(ctx, NT), dist(ctx, NT), daf(ctx, NT);
   Buffer<uint32_t> flags(ctx, NT);
-  Buffer<uint8_t> alive(ctx, NT);
   Buffer<unsigned long long> key(ctx, NT);
   fill_float(ctx, pdrf.data(), NT, INFINITY);
   fill_float(ctx, dist.data(), NT, INFINITY);
   fill_float(ctx, daf.data(), NT, INFINITY);
   flags.zero();
-  alive.zero();
   key.fill_bytes(0xFF);
-  // object voxel lists of all volumes at once (grouped by global object index), marking them alive
+  // object voxel lists of all volumes at once (grouped by global object index)
   std::vector<ArenaVolume> listed;
   std::vector<int> object_table;
   for (size_t v = 0; v < vs.size(); ++v) {
@@ -563,7 +561,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
     object_table.push_back(-1);
     object_table.push_back(vs[somas[j].volume].object_of[somas[j].id]);
   }
-  Buffer<int> vox = arena_object_voxels(ctx, ids.data(), NT, listed, object_table, nobj, F, alive.data());
+  Buffer<int> vox = arena_object_voxels(ctx, ids.data(), NT, listed, object_table, nobj, F);
   clock.mark("object_voxels");
   const size_t arenas = vs.size() + somas.size();
   std::vector<int> arena_offset(arenas), arena_dims(3 * arenas);
@@ -594,7 +592,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
     return n;
   };
   const int nbig_prepare = leading("BROOK_B200_PREPARE_CLUSTER_VOXELS",
-                                   tune.prepare_cluster_voxels > 0 ? tune.prepare_cluster_voxels : kPrepareClusterVoxels);
+                                   tune.prepare_cluster_voxels > 0 ? tune.prepare_cluster_voxels : prepare_cluster_voxels(F));
   const int nbig_trace = leading("BROOK_B200_TRACE_CLUSTER_VOXELS",
                                  tune.trace_cluster_voxels > 0 ? tune.trace_cluster_voxels : trace_cluster_voxels(F));
   auto d_arena_offset = to_device(ctx, arena_offset), d_arena_dims = to_device(ctx, arena_dims);
@@ -610,8 +608,8 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   auto d_rec_begin = to_device(ctx, rec_begin), d_rec_cap = to_device(ctx, rec_cap);
   Buffer<int> queue(ctx, 2), status(ctx, nobj), root(ctx, nobj), target(ctx, nobj), npaths(ctx, nobj), nstore(ctx, nobj);
   Buffer<float> max_daf(ctx, nobj);
-  Buffer<int> lists(ctx, 5 * F), store(ctx, store_total), rec_start(ctx, rec_total), rec_len(ctx, rec_total);
-  Buffer<unsigned long long> wide(ctx, F), side(ctx, 2 * F), work(ctx, 4), profile(ctx, 8LL * nobj);
+  Buffer<int> lists(ctx, 6 * F), store(ctx, store_total), rec_start(ctx, rec_total), rec_len(ctx, rec_total);
+  Buffer<unsigned long long> wide(ctx, F), work(ctx, 4), profile(ctx, 8LL * nobj);
   queue.zero();
   status.zero();
   work.zero();
@@ -619,10 +617,10 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   EngineArgs a{};
   a.arena_offset = d_arena_offset.data(); a.arena_dims = d_arena_dims.data(); a.obj_arena = d_obj_arena.data();
   a.mask = mask.data(); a.dbf = dbf.data(); a.pdrf = pdrf.data(); a.dist = dist.data(); a.daf = daf.data();
-  a.flags = flags.data(); a.alive = alive.data(); a.key = key.data();
+  a.flags = flags.data(); a.key = key.data(); a.n = unsigned(NT);
   a.nobj = nobj; a.obj_begin = d_obj_begin.data(); a.obj_count = d_obj_count.data(); a.vox = vox.data();
   a.schedule = d_schedule.data(); a.queue = queue.data(); a.status = status.data();
-  a.lists = lists.data(); a.wide = wide.data(); a.side = side.data(); a.F = F;
+  a.lists = lists.data(); a.wide = wide.data(); a.F = F;
   a.border_root = d_border_root.data(); a.M = d_M.data(); a.pdrf_scale = float(t.pdrf_scale); a.squarings = squarings;
   a.exponent = float(exponent);
   a.fix_branching = opt.fix_branching ? 1 : 0;
