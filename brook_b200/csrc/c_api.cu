@@ -646,10 +646,13 @@ brook_status brook_edt(brook_context *ctx, const brook_volume *labels, const flo
     handle->storage = std::make_shared<DeviceStorage>(size_t(n) * 4, ctx->value.device());
     handle->bytes = size_t(n) * 4;
     if (n) {
-      bk::Buffer<uint32_t> ids(ctx->value, n);
-      bk::connected_components(ctx->value, st.volume.data, st.volume.dtype, st.volume.d, ids.data());
-      bk::edt(ctx->value, ids.data(), st.volume.d, anisotropy, black_border != 0, 3,
-              static_cast<float *>(handle->storage->ptr));
+      float *out_field = static_cast<float *>(handle->storage->ptr);
+      bk::require_component_volume(st.volume.dtype, st.volume.d);
+      if (!bk::edt_labels(ctx->value, st.volume.data, st.volume.dtype, st.volume.d, anisotropy, black_border != 0, out_field)) {
+        bk::Buffer<uint32_t> ids(ctx->value, n);
+        bk::connected_components(ctx->value, st.volume.data, st.volume.dtype, st.volume.d, ids.data());
+        bk::edt(ctx->value, ids.data(), st.volume.d, anisotropy, black_border != 0, 3, out_field);
+      }
     }
     ctx->value.synchronize();
     handle->view = device_view(handle->storage->ptr, BROOK_F32, st.volume.d);

@@ -354,6 +354,13 @@ void for_dtype(int dtype, const void *labels, F &&f) {
 
 }  // namespace
 
+void require_component_volume(int dtype, VolumeDims d) {
+  label_bytes(dtype);  // rejects non-integer labels
+  if (d.n() >= (1LL << 31) - 1) throw std::invalid_argument("volumes of 2^31 voxels or more are not supported");
+  if ((d.sy + kTileY - 1) / kTileY > 65535 || (d.sz + kTileZ - 1) / kTileZ > 65535)
+    throw std::invalid_argument("volume too large for the tiled union");
+}
+
 std::vector<ComponentsResult> connected_components(Context &ctx, const std::vector<CcVolume> &volumes, uint32_t *ids,
                                                    bool planar) {
   std::vector<ComponentsResult> out(volumes.size());

@@ -3,8 +3,10 @@
 //   x: distance to the walls of each run of equal ids, from a float32 table of accumulated
 //      spacings (one rounding per step); one warp per x-line, coalesced, with run starts and ends
 //      found by warp max/min scans and the starts staged in shared memory;
-//   y, z: float64 lower envelope of parabolas per run, stored as float32; one thread per line,
-//      lines x-consecutive across a warp (coalesced), envelope stacks interleaved across lines;
+//   y, z: per run the least of height + squared spacing * squared steps, in float32 by scans over lines in
+//      shared memory where that gives the reference's float64 lower envelope of parabolas bit for bit
+//      (scan_is_exact), else by that envelope, one thread per line, lines x-consecutive across a warp
+//      (coalesced), envelope stacks interleaved across lines; stored as float32;
 //   the last pass takes the square root (background: 0).
 // The reference compiles the envelope with FMA contraction; its two product-plus-height sums are
 // written as explicit fused operations here, everything else rounds per operation (--fmad=false).
@@ -12,6 +14,7 @@
 #include <climits>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.hpp"
@@ -25,8 +28,10 @@ constexpr size_t kEdtXMaxSmem = 200 * 1024;
 
 // bb (here and in the envelope passes): walls beyond the line's ends, bit 0 before the first voxel,
 // bit 1 after the last (a black border sets both).
-__global__ void edt_x(const uint32_t *__restrict__ ids, float *__restrict__ D, Dims d, const float *__restrict__ acc,
-                      int bb, int finish) {
+template <class L>
+__global__ void edt_x(const L *__restrict__ ids, float *__restrict__ D, Dims d, const float *__restrict__ acc, int bb,
+                      int finish) {
+  using Id = std::conditional_t<sizeof(L) == 8, unsigned long long, uint32_t>;  // what a shuffle carries
   extern __shared__ int s_start[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long line = (long long)blockIdx.x * kWarpsX + warp;
@@ -35,12 +40,12 @@ __global__ void edt_x(const uint32_t *__restrict__ ids, float *__restrict__ D, D
   int *start = s_start + warp * sx;
   const long long base = line * sx;
   int carry_start = 0;
-  uint32_t carry_label = 0;
+  Id carry_label = 0;
   for (int c0 = 0; c0 < sx; c0 += 32) {
     const int p = c0 + lane;
     const bool in = p < sx;
-    const uint32_t lab = in ? ids[base + p] : 0xFFFFFFFFu;
-    uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, lab, 1);
+    const Id lab = in ? Id(ids[base + p]) : Id(0);
+    Id prev = __shfl_up_sync(0xFFFFFFFFu, lab, 1);
     if (lane == 0) prev = carry_label;
     int st = (in && (p == 0 || lab != prev)) ? p : -1;
 #pragma unroll
@@ -55,12 +60,12 @@ __global__ void edt_x(const uint32_t *__restrict__ ids, float *__restrict__ D, D
   }
   __syncwarp();
   int carry_end = sx - 1;
-  uint32_t carry_next = 0;
+  Id carry_next = 0;
   for (int c0 = ((sx - 1) / 32) * 32; c0 >= 0; c0 -= 32) {
     const int p = c0 + lane;
     const bool in = p < sx;
-    const uint32_t lab = in ? ids[base + p] : 0xFFFFFFFFu;
-    uint32_t next = __shfl_down_sync(0xFFFFFFFFu, lab, 1);
+    const Id lab = in ? Id(ids[base + p]) : Id(0);
+    Id next = __shfl_down_sync(0xFFFFFFFFu, lab, 1);
     if (lane == 31) next = carry_next;
     int en = (in && (p == sx - 1 || lab != next)) ? p : INT_MAX;
 #pragma unroll
@@ -94,7 +99,9 @@ void allow_edt_x_smem() {
   if (device < 0 || device >= 256) throw std::invalid_argument("device index out of range");
   std::lock_guard<std::mutex> guard(lock);
   if (raised[device]) return;
-  BK_CUDA(cudaFuncSetAttribute(edt_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEdtXMaxSmem));
+  for (const void *kernel : {(const void *)edt_x<uint8_t>, (const void *)edt_x<uint16_t>, (const void *)edt_x<uint32_t>,
+                             (const void *)edt_x<uint64_t>})
+    BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEdtXMaxSmem));
   raised[device] = true;
 }
 
@@ -269,6 +276,226 @@ __global__ void edt_envelope_volumes(const uint32_t *__restrict__ ids, float *__
   envelope_line(ids, D, base, stride, n, w, v.bb, Vs + tid, Hs + tid, Zs + tid, nbatch, finish);
 }
 
+// ---------------------------------------------------------------------------------------------
+// The y and z passes by bounded scans: a voxel's distance is the least of h(p) + w2 (q - p)^2 over its
+// run and of w2 j^2 to the run's walls, looked for outwards from q until w2 j^2 alone is no better.
+// Every value is one fused multiply-add in float32 (w2, j^2 and h are float32 values), that is the
+// exact sum rounded once, and rounding keeps the order, so the least rounded value is the rounded
+// least value. The envelope's float64 values are those sums too wherever scan_is_exact holds: its
+// numerators and products are then exact, and an intersection that is not a whole voxel lies farther
+// from it than the division rounds, so that each voxel is served by a parabola that is least there.
+//
+// A CTA holds 32 x-adjacent whole lines in shared memory (4 bytes a voxel: the height, whose sign bit
+// says that a run starts here; background: all ones), so the pass reads ids and heights once, writes once
+// and keeps no stacks in memory (the envelope's: 16 bytes a voxel written and read back). A lane owns
+// a column, so the banks never conflict. The scan is bound by its two shared loads a step; its length is
+// the distance found, a few voxels in segmentations. Past kNearSteps it goes by blocks of 32 voxels,
+// skipping those whose least height cannot improve (0 where a run starts in the block): solid volumes
+// cost n / 32 steps instead of n.
+constexpr int kScanCols = 32, kScanBlock = 32, kNearSteps = 24;
+constexpr unsigned kScanBackground = 0xFFFFFFFFu, kScanStart = 0x80000000u;
+constexpr size_t kScanMaxSmem = 220 * 1024;
+
+// A volume's tiles are [tile_begin, next tile_begin) of the launch's; bb as in the envelope passes.
+struct ScanVolume {
+  long long offset;
+  int tile_begin, sx, sy, sz, bb;
+  float w;
+};
+constexpr int kScanInline = 4;  // volumes described by the launch's parameters; more: by a table in memory
+struct ScanVolumes {
+  ScanVolume few[kScanInline];
+  const ScanVolume *many;
+  int count;
+};
+
+__host__ __device__ inline int scan_blocks(int n) { return (n + kScanBlock - 1) / kScanBlock; }
+inline size_t scan_smem(int n) { return size_t(n + scan_blocks(n)) * kScanCols * sizeof(float); }
+
+template <class L>
+__global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float *__restrict__ D,
+                                                const __grid_constant__ ScanVolumes vols, int axis, int finish) {
+  extern __shared__ unsigned s_line[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const ScanVolume *table = vols.many ? vols.many : vols.few;
+  int lo = 0, hi = vols.count - 1;  // the last volume whose first tile is at or before this one
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (table[mid].tile_begin <= int(blockIdx.x)) lo = mid; else hi = mid - 1;
+  }
+  const ScanVolume v = table[lo];
+  const int across = (v.sx + kScanCols - 1) / kScanCols, tile = int(blockIdx.x) - v.tile_begin;
+  const int x = (tile % across) * kScanCols + lane;
+  const long long rest = tile / across;  // z (y pass) or y (z pass)
+  const int n = axis == 1 ? v.sy : v.sz;
+  const long long stride = axis == 1 ? v.sx : (long long)v.sx * v.sy;
+  const long long base = v.offset + x + (axis == 1 ? (long long)v.sx * v.sy : (long long)v.sx) * rest;
+  const bool in = x < v.sx;
+  const int blocks = scan_blocks(n);
+  unsigned *column = s_line + lane;
+  float *least = reinterpret_cast<float *>(s_line + n * kScanCols) + lane;  // per block of the column
+  // a warp loads whole blocks of 32 rows, so that a row's previous id is in a register
+  for (int b = warp; b < blocks; b += warps) {
+    const int p0 = b * kScanBlock, p1 = min(n, p0 + kScanBlock);
+    L before = in && p0 > 0 ? ids[base + (p0 - 1) * stride] : L(0);
+    float m = __uint_as_float(BK_INF_BITS);
+#pragma unroll 8
+    for (int p = p0; p < p1; ++p) {
+      const L id = in ? ids[base + p * stride] : L(0);
+      const float h = in ? D[base + p * stride] : 0.0f;
+      const bool start = p == 0 || id != before;
+      before = id;
+      m = fminf(m, start ? 0.0f : h);
+      column[p * kScanCols] = id == 0 ? kScanBackground : (__float_as_uint(h) | (start ? kScanStart : 0u));
+    }
+    least[b * kScanCols] = m;
+  }
+  __syncthreads();
+  if (!in) return;
+  const float w2 = __fmul_rn(v.w, v.w);
+  for (int q = warp; q < n; q += warps) {
+    const unsigned own = column[q * kScanCols];
+    if (own == kScanBackground) {
+      if (finish) D[base + q * stride] = 0.0f;
+      continue;
+    }
+    float best = __uint_as_float(own & ~kScanStart);
+    // the low side goes on while the run started below the voxels seen, the high side until a start
+    bool low = true, high = true;
+    unsigned seen = own;
+    int j = 1;
+    for (; j <= kNearSteps && (low || high); ++j) {
+      const float jj = float(j * j), c = __fmul_rn(w2, jj);
+      if (c >= best) { low = high = false; break; }
+      if (low) {
+        const int p = q - j;
+        if (seen & kScanStart) {
+          if (p >= 0 || (v.bb & 1)) best = fminf(best, c);
+          low = false;
+        } else {
+          seen = column[p * kScanCols];
+          best = fminf(best, __fmaf_rn(w2, jj, __uint_as_float(seen & ~kScanStart)));
+        }
+      }
+      if (high) {
+        const int p = q + j;
+        const unsigned s = p < n ? column[p * kScanCols] : kScanStart;
+        if (s & kScanStart) {
+          if (p < n || (v.bb & 2)) best = fminf(best, c);
+          high = false;
+        } else best = fminf(best, __fmaf_rn(w2, jj, __uint_as_float(s)));
+      }
+    }
+    if (low)
+      for (int i = j;; ++i) {
+        const int p = q - i;
+        const float ii = float(i * i), c = __fmul_rn(w2, ii);
+        if (c >= best) break;
+        if (seen & kScanStart) {
+          if (p >= 0 || (v.bb & 1)) best = c;
+          break;
+        }
+        if ((p & (kScanBlock - 1)) == kScanBlock - 1 &&
+            __fmaf_rn(w2, ii, least[p / kScanBlock * kScanCols]) >= best) {
+          i += kScanBlock - 1;  // no start in the block: the run goes on below it
+          seen = 0;
+          continue;
+        }
+        seen = column[p * kScanCols];
+        best = fminf(best, __fmaf_rn(w2, ii, __uint_as_float(seen & ~kScanStart)));
+      }
+    if (high)
+      for (int i = j;; ++i) {
+        const int p = q + i;
+        const float ii = float(i * i), c = __fmul_rn(w2, ii);
+        if (c >= best) break;
+        if (p + kScanBlock <= n && (p & (kScanBlock - 1)) == 0 &&
+            __fmaf_rn(w2, ii, least[p / kScanBlock * kScanCols]) >= best) {
+          i += kScanBlock - 1;
+          continue;
+        }
+        const unsigned s = p < n ? column[p * kScanCols] : kScanStart;
+        if (s & kScanStart) {
+          if (p < n || (v.bb & 2)) best = c;
+          break;
+        }
+        best = fminf(best, __fmaf_rn(w2, ii, __uint_as_float(s)));
+      }
+    D[base + q * stride] = finish ? sqrtf(best) : best;
+  }
+}
+
+// Whether the scans give the envelope's values for spacings w and extents n (entries `axes` of each).
+// Every height and w2 is 0 or a float32 of at least the least squared spacing, so a whole multiple of
+// that square's last place g; sums stay below V. Numerators and products of the envelope are exact in 53
+// bits below V / g = 2^52, and an intersection lies on a whole voxel or at least g / (2 w2 n) from it,
+// which a division rounding at 2^-53 n resolves below 8 w2 n^2 / g = 2^53. (512 voxels an axis: spacings up
+// to 30 times apart, whatever their own digits.)
+bool scan_is_exact(const float *w, const int *n, int axes) {
+  double total = 0, last = INFINITY;
+  for (int a = 0; a < axes; ++a) {
+    const float w2 = w[a] * w[a];
+    if (!(w2 > 1e-30f) || !(w2 < 1e30f)) return false;
+    total += double(w2) * (double(n[a]) + 1) * (double(n[a]) + 1) * 1.01;  // 1.01: the x pass's accumulated spacings
+    last = std::min(last, std::ldexp(1.0, std::ilogb(w2) - 23));
+  }
+  return 16.0 * total < last * 9007199254740992.0;
+}
+
+// The line must fit a CTA's shared memory (1677 voxels); longer ones take the envelope.
+bool scan_fits(int n) { return scan_smem(n) <= kScanMaxSmem; }
+
+void allow_edt_scan_smem() {
+  static std::mutex lock;
+  static bool raised[256] = {};
+  int device = 0;
+  BK_CUDA(cudaGetDevice(&device));
+  if (device < 0 || device >= 256) throw std::invalid_argument("device index out of range");
+  std::lock_guard<std::mutex> guard(lock);
+  if (raised[device]) return;
+  for (const void *kernel : {(const void *)edt_scan<uint8_t>, (const void *)edt_scan<uint16_t>,
+                             (const void *)edt_scan<uint32_t>, (const void *)edt_scan<uint64_t>})
+    BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanMaxSmem));
+  raised[device] = true;
+}
+
+// Sets the volumes' tile_begin for a y (axis 1) or z (axis 2) pass; returns the launch's tiles.
+long long number_tiles(std::vector<ScanVolume> &vols, int axis, int &longest) {
+  long long tiles = 0;
+  longest = 1;
+  for (auto &v : vols) {
+    v.tile_begin = int(std::min<long long>(tiles, INT_MAX));
+    tiles += (long long)((v.sx + kScanCols - 1) / kScanCols) * (axis == 1 ? v.sz : v.sy);
+    longest = std::max(longest, axis == 1 ? v.sy : v.sz);
+  }
+  if (tiles > INT_MAX) throw std::invalid_argument("volume too large for the EDT scans");
+  return tiles;
+}
+
+template <class L>
+void launch_edt_scan(cudaStream_t s, const L *ids, float *D, std::vector<ScanVolume> &vols,
+                     const ScanVolume *many, long long tiles, int longest, int axis, int finish) {
+  ScanVolumes args{};
+  args.count = int(vols.size());
+  args.many = many;
+  if (!many) std::copy(vols.begin(), vols.end(), args.few);
+  allow_edt_scan_smem();
+  // 16 warps hide the loads of long lines; short ones have too few rows for them
+  edt_scan<<<unsigned(tiles), longest > 128 ? 512 : 256, scan_smem(longest), s>>>(ids, D, args, axis, finish);
+  BK_CUDA(cudaGetLastError());
+}
+
+template <class L>
+void edt_scan_pass(Context &ctx, const L *ids, float *D, std::vector<ScanVolume> vols, int axis, bool finish) {
+  int longest = 1;
+  const long long tiles = number_tiles(vols, axis, longest);
+  if (!tiles) return;
+  Buffer<ScanVolume> table;
+  if (vols.size() > size_t(kScanInline)) table = to_device(ctx, vols);
+  launch_edt_scan(ctx.stream(), ids, D, vols, table.data(), tiles, longest, axis, finish ? 1 : 0);
+  ++ctx.launches;
+}
+
 }  // namespace
 
 void edt(Context &ctx, const uint32_t *ids, VolumeDims vd, const float aniso[3], bool black_border, int dims,
@@ -292,8 +519,14 @@ void edt(Context &ctx, const uint32_t *ids, VolumeDims vd, const float aniso[3],
   edt_x<<<(unsigned)((xlines + kWarpsX - 1) / kWarpsX), kWarpsX * 32, smem, s>>>(ids, D, d, dacc.data(),
                                                                                 black_border ? 3 : 0, only_x ? 1 : 0); ++ctx.launches;
   BK_CUDA(cudaGetLastError());
+  const int extent[3] = {vd.sx, vd.sy, vd.sz};
+  const bool scans = scan_is_exact(aniso, extent, 3);
   for (int axis = 1; axis < dims; ++axis) {
-    const int len = axis == 1 ? vd.sy : vd.sz;
+    const int len = extent[axis];
+    if (scans && scan_fits(len)) {
+      edt_scan_pass(ctx, ids, D, {{0, 0, d.sx, d.sy, d.sz, black_border ? 3 : 0, aniso[axis]}}, axis, axis == dims - 1);
+      continue;
+    }
     const long long lines = axis == 1 ? (long long)vd.sx * vd.sz : (long long)vd.sx * vd.sy;
     const long long budget = 4LL << 30;  // bytes of envelope stacks per batch
     long long batch = std::max(1LL, std::min(lines, budget / (16LL * (len + 3))));
@@ -308,6 +541,43 @@ void edt(Context &ctx, const uint32_t *ids, VolumeDims vd, const float aniso[3],
       BK_CUDA(cudaGetLastError());
     }
   }
+}
+
+namespace {
+
+template <class L>
+void edt_of_labels(Context &ctx, const L *labels, Dims d, const float aniso[3], int bb, float *D) {
+  std::vector<float> acc(d.sx + 2, 0.0f);
+  for (size_t k = 1; k < acc.size(); ++k) acc[k] = acc[k - 1] + aniso[0];
+  Buffer<float> dacc = to_device(ctx, acc);
+  allow_edt_x_smem();
+  const long long xlines = (long long)d.sy * d.sz;
+  edt_x<<<(unsigned)((xlines + kWarpsX - 1) / kWarpsX), kWarpsX * 32, size_t(kWarpsX) * d.sx * sizeof(int),
+          ctx.stream()>>>(labels, D, d, dacc.data(), bb, 0);
+  ++ctx.launches;
+  BK_CUDA(cudaGetLastError());
+  for (int axis = 1; axis <= 2; ++axis)
+    edt_scan_pass(ctx, labels, D, {{0, 0, d.sx, d.sy, d.sz, bb, aniso[axis]}}, axis, axis == 2);
+}
+
+}  // namespace
+
+bool edt_labels(Context &ctx, const void *labels, int dtype, VolumeDims vd, const float aniso[3], bool black_border,
+                float *D) {
+  const int extent[3] = {vd.sx, vd.sy, vd.sz};
+  if (!scan_fits(vd.sy) || !scan_fits(vd.sz) || size_t(kWarpsX) * vd.sx * sizeof(int) > kEdtXMaxSmem) return false;
+  for (int a = 0; a < 3; ++a)
+    if (!(aniso[a] > 0) || !std::isfinite(aniso[a])) return false;
+  if (!scan_is_exact(aniso, extent, 3)) return false;
+  const Dims d{vd.sx, vd.sy, vd.sz};
+  const int bb = black_border ? 3 : 0;
+  switch (label_bytes(dtype)) {
+    case 1: edt_of_labels(ctx, static_cast<const uint8_t *>(labels), d, aniso, bb, D); break;
+    case 2: edt_of_labels(ctx, static_cast<const uint16_t *>(labels), d, aniso, bb, D); break;
+    case 4: edt_of_labels(ctx, static_cast<const uint32_t *>(labels), d, aniso, bb, D); break;
+    default: edt_of_labels(ctx, static_cast<const uint64_t *>(labels), d, aniso, bb, D); break;
+  }
+  return true;
 }
 
 void edt_xy_squared(Context &ctx, const uint32_t *ids, VolumeDims vd, const float aniso[3], bool black_border, float *D) {
@@ -378,6 +648,18 @@ void edt_planes(Context &ctx, const uint32_t *ids, int W, int H, int groups, int
   }
   BK_CUDA(cudaGetLastError());
   // the y pass of every group in one launch
+  bool scans = scan_fits(H);
+  std::vector<ScanVolume> stacks;
+  for (int g = 0; g < groups; ++g) {
+    const float spacing[2] = {wx[g], wy[g]};
+    const int extent[2] = {W, H};
+    scans = scans && scan_is_exact(spacing, extent, 2);
+    stacks.push_back({slice * per_group * g, 0, W, H, per_group, 3, wy[g]});
+  }
+  if (scans) {
+    edt_scan_pass(ctx, ids, D, std::move(stacks), 1, true);
+    return;
+  }
   const long long lines = (long long)W * S;
   const long long budget = 4LL << 30;
   const long long batch = std::max(1LL, std::min(lines, budget / (16LL * (H + 3))));
@@ -424,6 +706,18 @@ void edt_volumes(Context &ctx, const uint32_t *ids, const std::vector<EdtVolume>
   BK_CUDA(cudaGetLastError());
   // y and z passes: every volume's lines in one launch (a thread per line)
   for (int axis = 1; axis <= 2; ++axis) {
+    bool scans = true;
+    std::vector<ScanVolume> tiled;
+    for (const auto &v : vols) {
+      if (!v.d.n()) continue;
+      const int extent[3] = {v.d.sx, v.d.sy, v.d.sz};
+      scans = scans && scan_fits(extent[axis]) && scan_is_exact(aniso, extent, 3);
+      tiled.push_back({v.offset, 0, v.d.sx, v.d.sy, v.d.sz, walls(v, axis), aniso[axis]});
+    }
+    if (scans) {
+      edt_scan_pass(ctx, ids, D, std::move(tiled), axis, axis == 2);
+      continue;
+    }
     std::vector<EnvelopeVolume> table;
     long long lines = 0;
     int len = 1;
@@ -529,8 +823,17 @@ void edt_fixed_scratch(const uint32_t *labels, VolumeDims vd, const float aniso[
   edt_x<<<(unsigned)((xlines + kWarpsX - 1) / kWarpsX), kWarpsX * 32, smem, s>>>(labels, D, d, acc,
                                                                                 black_border ? 3 : 0, 0);
   BK_CUDA(cudaGetLastError());
+  const int extent[3] = {vd.sx, vd.sy, vd.sz};
+  const bool scans = scan_is_exact(aniso, extent, 3);
   for (int axis = 1; axis < 3; ++axis) {
-    const int len = axis == 1 ? vd.sy : vd.sz;
+    const int len = extent[axis];
+    if (scans && scan_fits(len)) {
+      std::vector<ScanVolume> volume{{0, 0, d.sx, d.sy, d.sz, black_border ? 3 : 0, aniso[axis]}};
+      int longest = 1;
+      const long long tiles = number_tiles(volume, axis, longest);
+      launch_edt_scan(s, labels, D, volume, nullptr, tiles, longest, axis, axis == 2);
+      continue;
+    }
     const long long lines = axis == 1 ? (long long)vd.sx * vd.sz : (long long)vd.sx * vd.sy;
     const long long room = (long long)((kFixedScratchBytes - table) / (16 * size_t(len + 3)));
     const long long batch = std::max(1LL, std::min(lines, room));

@@ -25,6 +25,8 @@ struct ComponentsResult {
   std::vector<int64_t> mapping;  // id -> original label (entry 0 unused), K + 1 entries
   std::vector<int64_t> roots;    // id - 1 -> first flat index of the component
 };
+// Throws where connected_components refuses a volume of these labels.
+void require_component_volume(int dtype, VolumeDims d);
 // 26-connected components of equal nonzero labels, ids by ascending first flat index, written to
 // ids (per voxel: id 1..K, 0 = background). `planar`: 8-connected within each z-slice only.
 ComponentsResult connected_components(Context &ctx, const void *labels, int dtype, VolumeDims d, uint32_t *ids,
@@ -60,6 +62,10 @@ void edt(Context &ctx, const uint32_t *ids, VolumeDims d, const float aniso[3], 
 // computed as edt() computes it, so the pieces give edt()'s field.
 void edt_xy_squared(Context &ctx, const uint32_t *ids, VolumeDims d, const float aniso[3], bool black_border, float *D);
 void edt_z_finish(Context &ctx, const uint32_t *ids, VolumeDims d, float wz, bool black_border, float *D);
+// The 3D EDT of integer labels without their components (runs of equal labels along a line are runs of one
+// component); false, with nothing done, where the y and z passes need the envelope.
+bool edt_labels(Context &ctx, const void *labels, int dtype, VolumeDims d, const float aniso[3], bool black_border,
+                float *D);
 struct EdtVolume {
   long long offset;
   VolumeDims d;

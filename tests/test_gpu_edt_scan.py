@@ -1,0 +1,58 @@
+"""The distance field's scans over whole lines against the oracle's envelope, bit for bit: lines at the edges of
+a block of 32 voxels and of the near steps, solid runs without a wall, columns that do not fill a tile, spacings on
+both sides of the rule that admits the scans, and a line too long for them."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _edt(labels, aniso, black_border):
+    from brook_b200 import _native as n
+
+    arr = ctypes.c_void_p()
+    vol = n.host_volume(labels)
+    n.check(n.load().brook_edt(n.context(0), ctypes.byref(vol), (ctypes.c_float * 3)(*aniso), int(black_border),
+                               ctypes.byref(arr)))
+    out = np.zeros(labels.shape, np.float32, order="F")
+    n.check(n.lib.brook_array_copy_to_host(arr, out.ctypes.data, out.nbytes))
+    n.lib.brook_array_destroy(arr)
+    return out
+
+
+def _labels(shape, kind):
+    rng = np.random.default_rng(sum(shape))
+    if kind == "solid":
+        return np.ones(shape, np.uint32, order="F")
+    if kind == "hole":  # one background voxel: nearly every voxel scans by blocks
+        v = np.ones(shape, np.uint32, order="F")
+        v[shape[0] // 2, shape[1] // 3, shape[2] - 1] = 0
+        return v
+    if kind == "noise":
+        return np.asfortranarray(rng.integers(0, 3, shape).astype(np.uint32))
+    # slabs of several labels, some over the volume's ends, with a few holes
+    v = (np.add.outer(np.add.outer(np.arange(shape[0]) // 19, np.arange(shape[1]) // 37), np.arange(shape[2]) // 29)
+         % 4).astype(np.uint32)
+    v[rng.random(shape) < 0.002] = 0
+    return np.asfortranarray(v)
+
+
+# (0.001, 1, 1000): the rule sends it to the envelope; (3.3, 0.7, 29.1): digits of its own
+@pytest.mark.parametrize("aniso", [(4, 4, 40), (1, 1, 1), (3.3, 0.7, 29.1), (0.001, 1, 1000)])
+@pytest.mark.parametrize("kind", ["solid", "hole", "noise", "slabs"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 31, 33), (33, 32, 64), (32, 25, 97), (70, 129, 1), (5, 24, 260)])
+def test_scans_match_oracle(gpu, shape, kind, aniso):
+    labels = _labels(shape, kind)
+    for black_border in (False, True):
+        np.testing.assert_array_equal(_edt(labels, aniso, black_border), oracle.edt(labels, aniso, black_border))
+
+
+def test_lines_past_shared_memory(gpu):
+    """1677 voxels fit a CTA's shared memory, 1678 take the envelope."""
+    for length in (1677, 1678):
+        labels = _labels((7, 2, length), "slabs")
+        np.testing.assert_array_equal(_edt(labels, (8, 8, 40), False), oracle.edt(labels, (8, 8, 40), False))
