@@ -158,17 +158,21 @@ __device__ __forceinline__ long long capped(const EngineArgs &a, long long bound
   return a.round_limit > 0 && a.round_limit < bound ? a.round_limit : bound;
 }
 
-// The queues' shared memory. Floods: two buffers of (voxel, distance bits) pairs. Invalidation: two
-// buffers of (voxel, key) pairs and the round's staged records. Four resident CTAs per SM then leave
-// half of the SM's 256 KB to L1, which holds the penalties.
-constexpr int kQueueBytes = 28672;
-constexpr int kFloodQueue = kQueueBytes / 16;   // pairs per buffer
-constexpr int kInvalQueue = kQueueBytes / 56;   // pairs per buffer, and records
-constexpr int kPipe = 2;  // frontier voxels a warp has in flight: their loads overlap
+// The queues' (dynamic) shared memory. Floods: two buffers of (voxel, distance bits) pairs. Invalidation:
+// two buffers of (voxel, key) pairs and the round's staged records.
+// One CTA is resident per SM, so the queues take what leaves L1 its half: 28 KB, which spilled a tenth of the
+// large objects' frontiers to HBM, cost 4 % of the 512^3 dense trace (28.5 -> 27.4 ms) and of an arbor's (37.7 ->
+// 36.1).
+constexpr int kQueueBytes = 96 * 1024;
+constexpr int kFloodQueue = kQueueBytes / 16;         // pairs per buffer
+constexpr int kInvalQueue = kQueueBytes / 56 / 2 * 2;  // pairs per buffer, and records
+// Frontier voxels a warp has in flight: their loads overlap. Three and four spill registers (512^3 dense trace
+// 27.4, 28.4, 29.9 ms with 2, 3 and 4).
+constexpr int kPipe = 2;
 
 __device__ __forceinline__ unsigned char *queue_bytes() {
-  __shared__ __align__(16) unsigned char buf[kQueueBytes];
-  return buf;
+  extern __shared__ __align__(16) unsigned char dynamic_queue[];
+  return dynamic_queue;
 }
 
 // This CTA's even share [lo, hi) of the entries that the group's CTAs hold in their queues, taken in
@@ -237,33 +241,36 @@ __device__ __forceinline__ void append(bool p, int v, int *list, int *count) {
   if (p) list[base + __popc(b & below(lane))] = v;
 }
 
-// Places in this CTA's queue `slot` and in two of the object's lists for what the lanes of a warp push
-// out of kPipe voxels' neighbourhoods: one counter atomic per list, the three at once, since each is a
-// round trip (to the group's first CTA for the lists).
+// Places in one list for what the lanes of a warp push out of kPipe voxels' neighbourhoods: the pushes'
+// ballots, and the list's next place (reserve), handed out voxel by voxel.
 struct Places {
-  int queue, touched, far;  // each list's next place; take() hands them out voxel by voxel
-  __device__ static int take(int &next, bool p) {
-    const unsigned b = __ballot_sync(kFull, p);
-    const int at = next + __popc(b & below(threadIdx.x & 31));
-    next += __popc(b);
+  unsigned ballot[kPipe];
+  int next;
+  __device__ int total() const {
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < kPipe; ++j) n += __popc(ballot[j]);
+    return n;
+  }
+  __device__ int take(int j) {  // this lane's place for voxel j, if it pushes there
+    const int at = next + __popc(ballot[j] & below(threadIdx.x & 31));
+    next += __popc(ballot[j]);
     return at;
   }
 };
 
-__device__ __forceinline__ Places reserve(const bool (&queued)[kPipe], const bool (&touched)[kPipe],
-                                          const bool (&far)[kPipe], int *queue_n, int *touched_n, int *far_n) {
+// One counter atomic per list, the three at once, since each is a round trip (to the group's first CTA
+// for the lists).
+__device__ __forceinline__ void reserve(Places &queued, Places &touched, Places &far, int *queue_n, int *touched_n,
+                                        int *far_n) {
   const int lane = threadIdx.x & 31;
-  int nq = 0, nt = 0, nf = 0;
-#pragma unroll
-  for (int j = 0; j < kPipe; ++j) {
-    nq += __popc(__ballot_sync(kFull, queued[j]));
-    nt += __popc(__ballot_sync(kFull, touched[j]));
-    nf += __popc(__ballot_sync(kFull, far[j]));
-  }
+  const int nq = queued.total(), nt = touched.total(), nf = far.total();
   const int n = lane == 0 ? nq : lane == 1 ? nt : lane == 2 ? nf : 0;
   int base = 0;
   if (n) base = atomicAdd(lane == 0 ? queue_n : lane == 1 ? touched_n : far_n, n);
-  return {__shfl_sync(kFull, base, 0), __shfl_sync(kFull, base, 1), __shfl_sync(kFull, base, 2)};
+  queued.next = __shfl_sync(kFull, base, 0);
+  touched.next = __shfl_sync(kFull, base, 1);
+  far.next = __shfl_sync(kFull, base, 2);
 }
 
 // A place in this CTA's next queue for each lane with p (at or past the queue's end: spill).
@@ -429,18 +436,19 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
         const bool want = neighbour && ((m[j] >> lane) & 1u) && du[j] >= x && cand[j] < dv[j];
         old[j] = want ? atomic_min_pos(d + int(e[j].x) + off, cand[j]) : -1.0f;
       }
-      int n = 0;
+      Places pushed;
 #pragma unroll
-      for (int j = 0; j < kPipe; ++j) n += __popc(__ballot_sync(kFull, old[j] > cand[j]));
+      for (int j = 0; j < kPipe; ++j) pushed.ballot[j] = __ballot_sync(kFull, old[j] > cand[j]);
+      const int n = pushed.total();
       if (!n) return;
       const int slot = (r + 1) % 3;
       int next = 0;
       if (lane == 0) next = atomicAdd(&sh.qn[slot], n);
-      next = __shfl_sync(kFull, next, 0);
+      pushed.next = __shfl_sync(kFull, next, 0);
 #pragma unroll
       for (int j = 0; j < kPipe; ++j) {
         const int v = int(e[j].x) + off;
-        const int q = Places::take(next, old[j] > cand[j]);
+        const int q = pushed.take(j);
         if (!(old[j] > cand[j])) continue;
         if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
         else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
@@ -550,9 +558,10 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
 // Every CTA belongs to a cluster. The clusters first take the large objects, one each, then every
 // CTA takes small objects on its own: large objects start first (they set the kernel's length),
 // and no CTA idles while any object is left.
+// (C == 1: a launch without large objects.)
 template <int C>
-__global__ void __launch_bounds__(kEngineThreads, 1) prepare_kernel(EngineArgs a) {
-  prepare_loop<C>(a, true);
+__global__ void __launch_bounds__(kEngineThreads, 1) prepare_kernel(const __grid_constant__ EngineArgs a) {
+  if constexpr (C > 1) prepare_loop<C>(a, true);
   prepare_loop<1>(a, false);
 }
 
@@ -644,34 +653,44 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
           const bool want = neighbour && ((m[j] >> lane) & 1u) && du[j] >= x && cand[j] < dv[j] && cand[j] <= nearest;
           old[j] = want ? atomic_min_pos(a.dist + int(e[j].x) + off, cand[j]) : -1.0f;
         }
-        bool near[kPipe], first[kPipe], beyond[kPipe], later[kPipe], any = false;
+        Places near, first, later;
+        unsigned beyond = 0;  // by voxel, this lane's
+        bool any = false;
 #pragma unroll
         for (int j = 0; j < kPipe; ++j) {
-          const bool improved = old[j] > cand[j], rail = rails && fv[j] == 0.0f;
-          first[j] = improved && old[j] == inf();
-          near[j] = improved && !rail && cand[j] <= T;
-          beyond[j] = improved && !rail && cand[j] > T;
-          later[j] = beyond[j] && first[j];
+          const bool improved = old[j] > cand[j], rail = rails && fv[j] == 0.0f, fresh = improved && old[j] == inf();
+          const bool far = improved && !rail && cand[j] > T;
+          near.ballot[j] = __ballot_sync(kFull, improved && !rail && !far);
+          first.ballot[j] = __ballot_sync(kFull, fresh);
+          later.ballot[j] = __ballot_sync(kFull, far && fresh);
+          beyond |= far ? 1u << j : 0u;
           any |= improved;
           if (improved && rail)
             atomicMin(&sh.rb, (static_cast<unsigned long long>(__float_as_uint(cand[j])) << 32) | unsigned(int(e[j].x) + off));
         }
         if (!__any_sync(kFull, any)) return;
         const int slot = (r + 1) % 3;
-        Places at = reserve(near, first, later, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
+        reserve(near, first, later, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
+        const bool defers = __any_sync(kFull, beyond);
 #pragma unroll
         for (int j = 0; j < kPipe; ++j) {
           const int v = int(e[j].x) + off;
-          const int q = Places::take(at.queue, near[j]);
-          if (near[j]) {
+          const int q = near.take(j);
+          if ((near.ballot[j] >> lane) & 1u) {
             if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
             else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
           }
-          const int w = Places::take(at.touched, first[j]);
-          if (first[j]) touched[w] = v;
-          const int f = Places::take(at.far, later[j]);
-          if (later[j]) far[f] = v;
-          if (__any_sync(kFull, beyond[j])) defer(beyond[j], cand[j], fv[j]);
+          const int w = first.take(j);
+          if ((first.ballot[j] >> lane) & 1u) touched[w] = v;
+          const int f = later.take(j);
+          if ((later.ballot[j] >> lane) & 1u) far[f] = v;
+        }
+        if (defers) {  // the lane's nearest of its voxels, then the warp's
+          float d = inf(), f = 0.0f;
+#pragma unroll
+          for (int j = 0; j < kPipe; ++j)
+            if (((beyond >> j) & 1u) && (cand[j] < d || (cand[j] == d && fv[j] < f))) { d = cand[j]; f = fv[j]; }
+          defer(beyond != 0, d, f);
         }
       };
       for (int i = s.lo + warp * kPipe; i < s.hi; i += warps * kPipe) {
@@ -967,6 +986,15 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
     append(claimed, v, touched, &L->n_touch);
   }
   G::sync();
+  auto stage = [&](int i, int u, int m, unsigned long long k) {
+    const int source = int(unsigned(k)) - 1;
+    const float rs = reach(a, source, sh.rscale, sh.rconst);
+    int x, y, z, qx, qy, qz;
+    coordinates(sh, u - sh.a0, x, y, z);
+    coordinates(sh, source - sh.a0, qx, qy, qz);
+    stage_id[i] = make_int4(u, m, source + 1, int(k >> 32));
+    stage_at[i] = make_float4(float(x - qx), float(y - qy), float(z - qz), rs);
+  };
   auto list_redo = [&](int v) {
     const int at = atomicAdd(&L->n_redo, 1);
     if (at < sh.count) redo[at] = v;
@@ -998,15 +1026,9 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
         if (i < s.hi) {
           const int u = of_rank<C>(queue_vox, q)[(r & 1) * kInvalQueue + at];
           const unsigned long long k = of_rank<C>(queue_key, q)[(r & 1) * kInvalQueue + at];
-          const int source = int(unsigned(k)) - 1;
           const unsigned m = a.mask[u];
           const bool current = __ldcg(a.key + u) == k;
-          const float rs = reach(a, source, sh.rscale, sh.rconst);
-          int x, y, z, qx, qy, qz;
-          coordinates(sh, u - sh.a0, x, y, z);
-          coordinates(sh, source - sh.a0, qx, qy, qz);
-          stage_id[i - s.lo] = make_int4(u, current ? int(m) : 0, source + 1, int(k >> 32));
-          stage_at[i - s.lo] = make_float4(float(x - qx), float(y - qy), float(z - qz), rs);
+          stage(i - s.lo, u, current ? int(m) : 0, k);
         }
       }
       for (int i = G::tid(); i < spilled; i += G::threads()) {
@@ -1015,81 +1037,73 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
         atomicAnd(a.flags + u, ~kFront);
       }
       G::sync();
-      // step B: a warp per voxel
-      auto offers = [&](const int4 (&e)[kPipe], const float4 (&at)[kPipe]) {
-        unsigned long long kv[kPipe], old[kPipe], cand[kPipe];
-        bool offer[kPipe];
+      // step B: a warp per voxel; the spilled voxels come after the queued ones, staged by this CTA
+      int staged = s.hi - s.lo;
+      for (int base = G::rank() * kInvalQueue;;) {
+        for (int i = warp * kPipe; i < staged; i += warps * kPipe) {
+          unsigned long long kv[kPipe], old[kPipe];
+          unsigned hb[kPipe];  // the offers' upper words
 #pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          const bool is = neighbour && ((unsigned(e[j].y) >> lane) & 1u);
-          kv[j] = is ? __ldcg(a.key + e[j].x + off) : 0ull;
-        }
-#pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          const float dx = __fmul_rn(a.wx, at[j].x + ox), dy = __fmul_rn(a.wy, at[j].y + oy),
-                      dz = __fmul_rn(a.wz, at[j].z + oz);
-          const float d = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-          const unsigned mb = max(__float_as_uint(d), unsigned(e[j].w));
-          cand[j] = (static_cast<unsigned long long>(mb < hi ? mb : mb | 0x80000000u) << 32) | unsigned(e[j].z);
-          offer[j] = d < at[j].w && cand[j] < kv[j];
-          old[j] = 0;
-          if (offer[j]) old[j] = atomicMin(a.key + e[j].x + off, cand[j]);
-        }
-        bool claimed[kPipe], first[kPipe], waits[kPipe], any = false;
-#pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          claimed[j] = old[j] > cand[j] && cand[j] < kWaits;
-          first[j] = claimed[j] && old[j] >= kWaits;
-          waits[j] = cand[j] >= kWaits && old[j] == BK_UNCLAIMED;
-          any |= claimed[j] || waits[j];
-          if (claimed[j] && !first[j]) list_redo(e[j].x + off);
-        }
-        if (!__any_sync(kFull, any)) return;
-        const int slot = (r + 1) % 3, buffer = ((r + 1) & 1) * kInvalQueue;
-        Places to = reserve(claimed, first, waits, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
-#pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          const int v = e[j].x + off;
-          const int q = Places::take(to.queue, claimed[j]);
-          if (claimed[j]) {
-            if (q < kInvalQueue) {
-              queue_vox[buffer + q] = v;
-              queue_key[buffer + q] = cand[j];
-            } else spill(a, v, kFront, nxt, &L->spilled[slot]);
+          for (int j = 0; j < kPipe; ++j) {
+            const int2 e = *reinterpret_cast<const int2 *>(stage_id + min(i + j, staged - 1));
+            const bool is = neighbour && i + j < staged && ((unsigned(e.y) >> lane) & 1u);
+            kv[j] = is ? __ldcg(a.key + e.x + off) : 0ull;
           }
-          const int w = Places::take(to.touched, first[j]);
-          if (first[j]) touched[w] = v;
-          const int f = Places::take(to.far, waits[j]);
-          if (waits[j]) far[f] = v;
-        }
-      };
-      const int staged = s.hi - s.lo;
-      for (int i = warp * kPipe; i < staged; i += warps * kPipe) {
-        int4 e[kPipe];
-        float4 at[kPipe];
 #pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          e[j] = stage_id[min(i + j, staged - 1)];
-          at[j] = stage_at[min(i + j, staged - 1)];
-          if (i + j >= staged) e[j].y = 0;
-        }
-        offers(e, at);
-      }
-      for (int i = (G::tid() >> 5) * kPipe; i < spilled; i += (G::threads() >> 5) * kPipe) {
-        int4 e[kPipe];
-        float4 at[kPipe];
+          for (int j = 0; j < kPipe; ++j) {
+            const int4 e = stage_id[min(i + j, staged - 1)];
+            const float4 at = stage_at[min(i + j, staged - 1)];
+            const float dx = __fmul_rn(a.wx, at.x + ox), dy = __fmul_rn(a.wy, at.y + oy), dz = __fmul_rn(a.wz, at.z + oz);
+            const float d = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+            const unsigned mb = max(__float_as_uint(d), unsigned(e.w));
+            hb[j] = mb < hi ? mb : mb | 0x80000000u;
+            const unsigned long long cand = (static_cast<unsigned long long>(hb[j]) << 32) | unsigned(e.z);
+            old[j] = 0;
+            if (d < at.w && cand < kv[j]) old[j] = atomicMin(a.key + e.x + off, cand);
+          }
+          Places claimed, first, waits;
+          unsigned any = 0;
 #pragma unroll
-        for (int j = 0; j < kPipe; ++j) {
-          const int w = min(i + j, spilled - 1), u = __ldcg(cur + w);
-          const unsigned long long k = __ldcg(wide + w);
-          const int source = int(unsigned(k)) - 1;
-          int x, y, z, qx, qy, qz;
-          coordinates(sh, u - sh.a0, x, y, z);
-          coordinates(sh, source - sh.a0, qx, qy, qz);
-          e[j] = make_int4(u, i + j < spilled ? int(a.mask[u]) : 0, source + 1, int(k >> 32));
-          at[j] = make_float4(float(x - qx), float(y - qy), float(z - qz), reach(a, source, sh.rscale, sh.rconst));
+          for (int j = 0; j < kPipe; ++j) {
+            const int4 e = stage_id[min(i + j, staged - 1)];
+            const unsigned long long cand = (static_cast<unsigned long long>(hb[j]) << 32) | unsigned(e.z);
+            const bool claims = old[j] > cand && cand < kWaits;
+            claimed.ballot[j] = __ballot_sync(kFull, claims);
+            first.ballot[j] = __ballot_sync(kFull, claims && old[j] >= kWaits);
+            waits.ballot[j] = __ballot_sync(kFull, cand >= kWaits && old[j] == BK_UNCLAIMED);
+            any |= claimed.ballot[j] | waits.ballot[j];
+            if (claims && old[j] < kWaits) list_redo(e.x + off);
+          }
+          if (!any) continue;
+          const int slot = (r + 1) % 3, buffer = ((r + 1) & 1) * kInvalQueue;
+          reserve(claimed, first, waits, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
+#pragma unroll
+          for (int j = 0; j < kPipe; ++j) {
+            const int4 e = stage_id[min(i + j, staged - 1)];
+            const int v = e.x + off;
+            const int q = claimed.take(j);
+            if ((claimed.ballot[j] >> lane) & 1u) {
+              if (q < kInvalQueue) {
+                queue_vox[buffer + q] = v;
+                queue_key[buffer + q] = (static_cast<unsigned long long>(hb[j]) << 32) | unsigned(e.z);
+              } else spill(a, v, kFront, nxt, &L->spilled[slot]);
+            }
+            const int w = first.take(j);
+            if ((first.ballot[j] >> lane) & 1u) touched[w] = v;
+            const int f = waits.take(j);
+            if ((waits.ballot[j] >> lane) & 1u) far[f] = v;
+          }
         }
-        offers(e, at);
+        if (base >= spilled) break;
+        __syncthreads();  // the records are free
+        staged = min(kInvalQueue, spilled - base);
+        for (int i = threadIdx.x; i < staged; i += blockDim.x) {
+          const int u = __ldcg(cur + base + i);
+          const unsigned long long k = __ldcg(wide + base + i);
+          stage(i, u, int(a.mask[u]), k);
+        }
+        base += C * kInvalQueue;
+        __syncthreads();
       }
       G::sync();
     }
@@ -1186,8 +1200,10 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
   return true;
 }
 
+// A function of its own: inlined into a kernel of lone CTAs the same loop took 33.1 ms of the 512^3 dense
+// trace and 23.3 as a call, on the same 148 CTAs (64 registers either way).
 template <int C>
-__device__ void trace_loop(const EngineArgs &a, bool big) {
+__device__ __noinline__ void trace_loop(const EngineArgs &a, bool big) {
   using G = Group<C>;
   __shared__ Shared sh;
   __shared__ unsigned long long s_work[4];
@@ -1378,12 +1394,14 @@ __device__ void trace_loop(const EngineArgs &a, bool big) {
   if (threadIdx.x < 4 && s_work[threadIdx.x]) atomicAdd(a.work + threadIdx.x, s_work[threadIdx.x]);
 }
 
-template <int C>
 // The first a.lone_first clusters start on the small objects (each CTA alone, largest first) and
 // then join the large ones; the others take the large objects first. So the longest lone-CTA
-// objects run beside the clusters' objects from the start instead of after them.
-__global__ void __launch_bounds__(kEngineThreads, 1) trace_kernel(EngineArgs a) {
-  if (int(blockIdx.x) / C < a.lone_first) {
+// objects run beside the clusters' objects from the start instead of after them. (C == 1: a launch
+// without large objects.)
+template <int C>
+__global__ void __launch_bounds__(kEngineThreads, 1) trace_kernel(const __grid_constant__ EngineArgs a) {
+  if constexpr (C == 1) trace_loop<1>(a, false);
+  else if (int(blockIdx.x) / C < a.lone_first) {
     trace_loop<1>(a, false);
     trace_loop<C>(a, true);
   } else {
@@ -1396,6 +1414,7 @@ cudaLaunchConfig_t cluster_config(int clusters, int ctas, cudaStream_t stream, c
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(unsigned(clusters * ctas));
   config.blockDim = dim3(kEngineThreads);
+  config.dynamicSmemBytes = kQueueBytes;
   config.stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = unsigned(ctas);
@@ -1416,6 +1435,8 @@ int resident_clusters(const void *kernel, int ctas, cudaStream_t stream) {
   std::lock_guard<std::mutex> guard(lock);
   auto it = known.find({device, kernel});
   if (it != known.end()) return it->second;
+  // once per device and kernel, before its first launch
+  BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQueueBytes));
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t probe = cluster_config(1, ctas, stream, attr);
   int cap = 1;
@@ -1433,7 +1454,7 @@ void launch(const void *kernel, int ctas, const EngineArgs &a, int nbig, cudaStr
   const int cap = std::max(1, resident_clusters(kernel, ctas, stream) * std::min(100, std::max(1, a.grid_percent)) / 100);
   const long long need = nbig + (a.nobj - nbig + ctas - 1) / ctas;
   const int clusters = int(std::max(1LL, std::min<long long>(cap, need)));
-  args.lone_first = nbig < a.nobj ? clusters * lone_percent / 100 : 0;
+  args.lone_first = nbig > 0 && nbig < a.nobj ? clusters * lone_percent / 100 : 0;
   cudaLaunchConfig_t config = cluster_config(clusters, ctas, stream, attr);
   BK_CUDA(cudaLaunchKernelExC(&config, kernel, kargs));
 }
@@ -1451,39 +1472,55 @@ static long long resident_ctas() {
   if (it == known.end()) {
     int sms = 1, per_sm = 1;
     BK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas>, kEngineThreads, 0));
+    BK_CUDA(cudaFuncSetAttribute(trace_kernel<kClusterCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQueueBytes));
+    BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas>, kEngineThreads, kQueueBytes));
     it = known.emplace(device, std::max(1LL, (long long)sms * per_sm)).first;
   }
   return it->second;
 }
 
 long long trace_cluster_voxels(long long foreground) {
-  return std::max(kTraceClusterFloor, foreground / resident_ctas());
+  return std::max(kTraceClusterFloor, foreground / resident_ctas() * 3 / 2);
 }
 
 long long prepare_cluster_voxels(long long foreground) {
-  return std::max(kPrepareClusterFloor, foreground / (2 * resident_ctas()));
+  const long long share = foreground / resident_ctas();
+  return std::max(kPrepareClusterFloor, share >= kPrepareWholeShare ? share : share / 2);
 }
 
 int cluster_ctas(long long largest, long long foreground) {
   return largest * kWideClusterShare >= foreground ? kWideClusterCtas : kClusterCtas;
 }
 
-void launch_prepare(const EngineArgs &a, int nbig, int ctas, cudaStream_t stream) {
-  if (ctas == kWideClusterCtas) launch((const void *)prepare_kernel<kWideClusterCtas>, ctas, a, nbig, stream);
-  else launch((const void *)prepare_kernel<kClusterCtas>, kClusterCtas, a, nbig, stream);
+// The kernel for nbig large objects. Without any, CTAs are launched alone: clusters of 4 fit only 132 of the 148
+// SMs, since an SM short of a whole cluster in its part of the chip stays idle.
+static const void *prepare_variant(int nbig, int &ctas) {
+  if (nbig == 0) { ctas = 1; return (const void *)prepare_kernel<1>; }
+  if (ctas == kWideClusterCtas) return (const void *)prepare_kernel<kWideClusterCtas>;
+  ctas = kClusterCtas;
+  return (const void *)prepare_kernel<kClusterCtas>;
+}
+static const void *trace_variant(int nbig, int &ctas) {
+  if (nbig == 0) { ctas = 1; return (const void *)trace_kernel<1>; }
+  if (ctas == kWideClusterCtas) return (const void *)trace_kernel<kWideClusterCtas>;
+  ctas = kClusterCtas;
+  return (const void *)trace_kernel<kClusterCtas>;
 }
 
-void prepare_engine_launches(int prepare_ctas, int trace_ctas, cudaStream_t stream) {
-  if (prepare_ctas == kWideClusterCtas) resident_clusters((const void *)prepare_kernel<kWideClusterCtas>, kWideClusterCtas, stream);
-  else resident_clusters((const void *)prepare_kernel<kClusterCtas>, kClusterCtas, stream);
-  if (trace_ctas == kWideClusterCtas) resident_clusters((const void *)trace_kernel<kWideClusterCtas>, kWideClusterCtas, stream);
-  else resident_clusters((const void *)trace_kernel<kClusterCtas>, kClusterCtas, stream);
+void launch_prepare(const EngineArgs &a, int nbig, int ctas, cudaStream_t stream) {
+  const void *kernel = prepare_variant(nbig, ctas);
+  launch(kernel, ctas, a, nbig, stream);
+}
+
+void prepare_engine_launches(int nbig_prepare, int prepare_ctas, int nbig_trace, int trace_ctas, cudaStream_t stream) {
+  const void *prepare = prepare_variant(nbig_prepare, prepare_ctas), *trace = trace_variant(nbig_trace, trace_ctas);
+  resident_clusters(prepare, prepare_ctas, stream);
+  resident_clusters(trace, trace_ctas, stream);
 }
 
 void launch_trace(const EngineArgs &a, int nbig, int ctas, int lone_percent, cudaStream_t stream) {
-  if (ctas == kWideClusterCtas) launch((const void *)trace_kernel<kWideClusterCtas>, ctas, a, nbig, stream, lone_percent);
-  else launch((const void *)trace_kernel<kClusterCtas>, kClusterCtas, a, nbig, stream, lone_percent);
+  const void *kernel = trace_variant(nbig, ctas);
+  launch(kernel, ctas, a, nbig, stream, lone_percent);
 }
 
 }  // namespace bk

@@ -120,17 +120,18 @@ constexpr int kClusterCtas = 4;
 constexpr int kWideClusterCtas = 8;
 constexpr long long kWideClusterShare = 16;
 int cluster_ctas(long long largest, long long foreground);
-// Tracing: the foreground voxels per resident CTA, at least kTraceClusterFloor. Measured (trace ms with
-// clusters from 2048, 16384 and 65536 voxels, and without): 512^3 dense (share 190 k) 79.0, 71.7,
-// 43.1, 29.7; 16 volumes in a batch (56 k) 33.5, 24.9, 10.0, 9.7; 256^3 dense (24 k) 11.8, 11.7, 11.6,
-// 17.8; 128^3 tubes (3 k; objects up to 61 k) 7.9, 7.8, 9.1, 9.1; a 48^3 request (objects of 16-31 k)
-// 4.9, 4.9, 4.1, 4.1.
+// Tracing: one and a half shares of the foreground voxels per resident CTA, at least kTraceClusterFloor.
+// Measured (trace ms by the objects' least voxels for a cluster): 512^3 dense (share 190 k) 64 from 30 k, 45 from
+// 60 k, 23.3 without; 16 volumes in a batch (56 k) 17.8 from 30 k, 10.4 from 56 k, 8.2 from 80 k, 7.9 from 160 k;
+// 256^3 dense (24 k) 11.7 from 33 k and from 80 k, 13.7 from 160 k; 128^3 tubes (3 k; objects up to 61 k) 8.9 from
+// 33 k, 9.5 from 80 k; a 48^3 request (objects of 16-31 k) 3.1 at each.
 constexpr long long kTraceClusterFloor = 32768;
 long long trace_cluster_voxels(long long foreground);
-// Preparation, whose floods have frontiers ten times as wide: half that share, at least
-// kPrepareClusterFloor (prepare ms, the same columns: 20.9, 18.3, 14.4, 12.9; 6.4, 4.8, 3.9, 4.1; 2.6, 2.9,
-// 5.1, 6.2; 1.2, 1.1, 2.6, 2.5; 0.48, 0.61, 1.1, 1.1).
-constexpr long long kPrepareClusterFloor = 4096;
+// Preparation, whose floods have frontiers ten times as wide: the share from kPrepareWholeShare on, below it
+// half the share, at least kPrepareClusterFloor (prepare ms): 512^3 dense 17.8 from 20 k, 14.6 from 60 k, 13.0
+// from 100 k, 11.4 without; the batch 4.0 from 28 k, 3.1 from 56 k, 4.0 without; 256^3 dense 2.3 from 12 k, 2.7
+// from 20 k, 4.5 from 60 k.
+constexpr long long kPrepareClusterFloor = 4096, kPrepareWholeShare = 32768;
 long long prepare_cluster_voxels(long long foreground);
 
 // One pass of the engine: clusters take schedule[0, nbig) (large objects, largest first), then
@@ -145,6 +146,7 @@ constexpr int kLoneFirstPercent = 10;
 constexpr float kRailBand = 0.5f;
 // The device queries the launches above make (resident clusters per kernel), done ahead so that
 // a stream capture of the launches holds launches only.
-void prepare_engine_launches(int prepare_cluster_ctas, int trace_cluster_ctas, cudaStream_t stream);
+void prepare_engine_launches(int nbig_prepare, int prepare_cluster_ctas, int nbig_trace, int trace_cluster_ctas,
+                             cudaStream_t stream);
 
 }  // namespace bk

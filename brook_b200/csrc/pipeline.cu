@@ -692,7 +692,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   };
   if (as_graph) {
     const auto graph_start = std::chrono::steady_clock::now();
-    prepare_engine_launches(prepare_ctas, ctas, s);  // device queries, before the capture
+    prepare_engine_launches(nbig_prepare, prepare_ctas, nbig_trace, ctas, s);  // device queries, before the capture
     BK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     clock.capturing(true);
     try {
