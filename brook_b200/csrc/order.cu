@@ -1,16 +1,16 @@
-// Object voxel lists and target orders, with CUB's device sorts:
+// Object voxel lists and target orders, with CUB's radix sorts:
 //  * the voxels of every object of every volume of a call, grouped by object and ascending in
 //    flat index (one compaction of the arena in flat order and one stable radix sort by object);
 //  * per object the target order: descending DAF (infinite -> 0), ties -> higher flat index first
 //    (lockstep_order.cu:21-45 of giorgioangel/brook). Inside an object the voxel list ascends in
-//    flat index, so "higher flat first" is "later list position first": the composite key
-//    (object rank, 0x7FFFFFFF - DAF bits, last position - position) orders every object at once in
-//    one device-wide radix sort over all SMs (a non-negative float's sign bit is 0, so 31 DAF bits
-//    suffice). The key is a 64-bit word when the object, DAF and position bits fit, else a
-//    (32-bit, 64-bit) pair sorted through a decomposer over only the bits in use.
+//    flat index, so "higher flat first" is "later list position first". One device-wide radix sort over all
+//    SMs orders every object at once: by (object, DAF) with the position as payload of a 64-bit key where
+//    the three fit, else by (object, DAF, position) in a (32-bit, 64-bit) pair sorted through a decomposer over
+//    only the bits in use (a non-negative float's sign bit is 0, so at most 31 DAF bits).
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
+
+#include <cstring>
 
 #include "order.hpp"
 
@@ -79,12 +79,20 @@ __device__ __forceinline__ unsigned long long order_low(const int *vox, const fl
          (lmask - unsigned(i - __ldg(begin + o)));
 }
 
-__global__ void order_keys64(const int *vox, const float *daf, const int *begin, int nobj, int lbits,
-                             unsigned long long *keys, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// The 64-bit key: o << (lbits + dbits) | (distance from the call's largest possible DAF) << lbits | position in o,
+// in descending list order, so that a stable sort of the upper two fields alone leaves ties in that order.
+__global__ void order_keys64(const int *vox, const float *daf, const int *begin, int nobj, int lbits, int dbits,
+                             unsigned top, unsigned long long *keys, int n) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int i = n - 1 - j;
   const int o = object_of_position(begin, nobj, i);
-  keys[i] = (static_cast<unsigned long long>(o) << (lbits + 31)) | order_low(vox, daf, begin, o, i, lbits);
+  const float d = daf[vox[i]];
+  const unsigned last = (1u << dbits) - 1;
+  // 0 (and infinite) comes last; the positive values are within [top - last + 1, top] (order_bits)
+  const unsigned field = isinf(d) || d == 0.0f ? last : min(top - min(__float_as_uint(d), top), last - 1);
+  keys[j] = (static_cast<unsigned long long>(o) << (lbits + dbits)) | (static_cast<unsigned long long>(field) << lbits) |
+            unsigned(i - __ldg(begin + o));
 }
 
 __global__ void order_keys96(const int *vox, const float *daf, const int *begin, int nobj, int lbits, WideKey *keys,
@@ -105,12 +113,12 @@ __device__ __forceinline__ int order_voxel(const int *vox, const int *begin, int
   return vox[__ldg(begin + o) + int(lmask - (lo & lmask))];
 }
 
-__global__ void unpack_order64(const unsigned long long *keys, const int *vox, const int *begin, int lbits, int *order,
-                               int n) {
+__global__ void unpack_order64(const unsigned long long *keys, const int *vox, const int *begin, int lbits, int dbits,
+                               int *order, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long k = keys[i];
-  order[i] = order_voxel(vox, begin, int(k >> (lbits + 31)), k, lbits);
+  order[i] = vox[__ldg(begin + int(k >> (lbits + dbits))) + int(k & ((1ULL << lbits) - 1))];
 }
 
 __global__ void unpack_order96(const WideKey *keys, const int *vox, const int *begin, int lbits, int *order, int n) {
@@ -171,7 +179,24 @@ Buffer<int> arena_object_voxels(Context &ctx, const uint32_t *ids, long long n, 
   return vox;
 }
 
-OrderPlan plan_target_orders(Context &ctx, long long total, int nobj, long long largest, bool wide) {
+// The bits of a DAF's field in the 64-bit key, and the float bits of a bound that no finite DAF passes. A
+// positive DAF is at least one step (half of it allows for the free-space seed's roundings) and at most one step
+// per voxel of the largest object, each sum rounded up by 2^-24 of itself at most (a doubling below 2^23 voxels).
+void order_bits(long long largest, float least_step, float most_step, int &bits, unsigned &top) {
+  const float lower = 0.5f * least_step, upper = 2.0f * most_step * float(largest);
+  bits = 31;
+  top = 0x7FFFFFFFu;
+  // spacings 1e4 times apart: a seed's roundings stay below its half step
+  if (largest >= (1LL << 23) || !(most_step < 1e4f * least_step) || !(lower > 0.0f) || !(upper < INFINITY) || !(upper > lower)) return;
+  unsigned low = 0;
+  std::memcpy(&low, &lower, sizeof(low));
+  std::memcpy(&top, &upper, sizeof(top));
+  bits = 1;
+  while ((1ULL << bits) < (unsigned long long)(top - low) + 2) ++bits;
+}
+
+OrderPlan plan_target_orders(Context &ctx, long long total, int nobj, long long largest, float least_step,
+                             float most_step, bool wide) {
   OrderPlan p;
   p.total = total;
   p.nobj = nobj;
@@ -183,15 +208,18 @@ OrderPlan plan_target_orders(Context &ctx, long long total, int nobj, long long 
     return b;
   };
   p.lbits = bits_for(largest);
+  order_bits(largest, least_step, most_step, p.dbits, p.top);
   p.end_bit = p.lbits + 31 + bits_for(nobj);
   p.wide = wide || p.end_bit > 64;
+  // the position is a payload of the 64-bit key. 512^3 dense: 39 sorted bits of 60, 5 passes instead of 8
+  if (!p.wide) p.end_bit = p.lbits + p.dbits + bits_for(nobj);
   const size_t key_bytes = p.wide ? sizeof(WideKey) : sizeof(unsigned long long);
   p.keys = Buffer<unsigned char>(ctx, total * key_bytes);
   p.sorted = Buffer<unsigned char>(ctx, total * key_bytes);
   // the scratch size is a host computation (no stream work)
   if (!p.wide)
     BK_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, p.temp, reinterpret_cast<unsigned long long *>(p.keys.data()),
-                                           reinterpret_cast<unsigned long long *>(p.sorted.data()), (int)total, 0,
+                                           reinterpret_cast<unsigned long long *>(p.sorted.data()), (int)total, p.lbits,
                                            p.end_bit, ctx.stream()));
   else
     BK_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, p.temp, reinterpret_cast<WideKey *>(p.keys.data()),
@@ -209,11 +237,11 @@ void run_target_orders(Context &ctx, OrderPlan &p, const int *vox, const float *
   if (!p.wide) {
     auto *keys = reinterpret_cast<unsigned long long *>(p.keys.data());
     auto *sorted = reinterpret_cast<unsigned long long *>(p.sorted.data());
-    order_keys64<<<blocks_for(total), 256, 0, s>>>(vox, daf, begin, p.nobj, p.lbits, keys, (int)total);
+    order_keys64<<<blocks_for(total), 256, 0, s>>>(vox, daf, begin, p.nobj, p.lbits, p.dbits, p.top, keys, (int)total);
     ++ctx.launches;
     BK_CUDA(cudaGetLastError());
-    BK_CUDA(cub::DeviceRadixSort::SortKeys(p.scratch.data(), temp, keys, sorted, (int)total, 0, p.end_bit, s));
-    unpack_order64<<<blocks_for(total), 256, 0, s>>>(sorted, vox, begin, p.lbits, p.order.data(), (int)total);
+    BK_CUDA(cub::DeviceRadixSort::SortKeys(p.scratch.data(), temp, keys, sorted, (int)total, p.lbits, p.end_bit, s));
+    unpack_order64<<<blocks_for(total), 256, 0, s>>>(sorted, vox, begin, p.lbits, p.dbits, p.order.data(), (int)total);
   } else {
     auto *keys = reinterpret_cast<WideKey *>(p.keys.data());
     auto *sorted = reinterpret_cast<WideKey *>(p.sorted.data());
@@ -226,13 +254,6 @@ void run_target_orders(Context &ctx, OrderPlan &p, const int *vox, const float *
   }
   ++ctx.launches;
   BK_CUDA(cudaGetLastError());
-}
-
-Buffer<int> target_orders(Context &ctx, const int *vox, const float *daf, long long total, const int *begin, int nobj,
-                          long long largest, bool wide) {
-  OrderPlan p = plan_target_orders(ctx, total, nobj, largest, wide);
-  run_target_orders(ctx, p, vox, daf, begin);
-  return std::move(p.order);
 }
 
 }  // namespace bk

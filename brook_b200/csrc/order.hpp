@@ -17,7 +17,7 @@ Buffer<int> arena_object_voxels(Context &ctx, const uint32_t *ids, long long n, 
                                 const std::vector<int> &object_of, int nobj, long long total);
 // Per object (voxels [begin[o], begin[o+1]) of the list, the last to `total`): its voxels by
 // descending DAF (inf -> 0), ties -> higher flat first. `largest` is the largest object's voxel
-// count; `wide` forces the (32, 64)-bit key even where 64 bits would hold it.
+// count and a step of a DAF is within [least_step, most_step]; `wide` forces the (32, 64)-bit key even where 64 bits would hold it.
 // In two steps: plan_target_orders makes every buffer (no stream work), run_target_orders only
 // launches, so that a stream capture of it holds kernels and no allocations.
 struct OrderPlan {
@@ -25,11 +25,11 @@ struct OrderPlan {
   Buffer<unsigned char> keys, sorted, scratch;
   size_t temp = 0;
   long long total = 0;
-  int nobj = 0, lbits = 0, end_bit = 0;
+  int nobj = 0, lbits = 0, dbits = 31, end_bit = 0;
+  unsigned top = 0;  // float bits that no finite DAF passes
   bool wide = false;
 };
-OrderPlan plan_target_orders(Context &ctx, long long total, int nobj, long long largest, bool wide = false);
+OrderPlan plan_target_orders(Context &ctx, long long total, int nobj, long long largest, float least_step,
+                             float most_step, bool wide = false);
 void run_target_orders(Context &ctx, OrderPlan &plan, const int *vox, const float *daf, const int *begin);
-Buffer<int> target_orders(Context &ctx, const int *vox, const float *daf, long long total, const int *begin, int nobj,
-                          long long largest, bool wide = false);
 }  // namespace bk

@@ -664,7 +664,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   lone_percent = std::max(0, std::min(100, lone_percent));
   const char *fields = std::getenv("BROOK_B200_DUMP_FIELDS");
   const bool wide_order = std::getenv("BROOK_B200_WIDE_ORDER_KEY") != nullptr;  // test knob: the 96-bit key path
-  OrderPlan orders = plan_target_orders(ctx, F, nobj, largest, wide_order);
+  OrderPlan orders = plan_target_orders(ctx, F, nobj, largest, a.delta, a.w[25], wide_order);
   a.order = orders.order.data();
   // the engine's launches, prepare -> target orders -> trace, as one CUDA graph (every buffer is
   // made above; the graph holds kernels, a memset and the stage marks): one submission per call,
