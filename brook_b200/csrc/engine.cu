@@ -375,13 +375,22 @@ __device__ float freespace_seed(const EngineArgs &a, int x, int y, int z, int rx
 // A round waits for two dependent L2 round trips (the neighbours' distances, then the atomic
 // minimum of those that improve) and one group barrier. A queued pair whose voxel has a smaller
 // distance by now is skipped: that distance has been queued too.
+// A lone CTA's flood goes by bands: distances past the band's end T only enter the far list, at their first
+// touch; when the band has converged the list's voxels become the frontier, each with the least of the offers it
+// got meanwhile. Without bands a voxel was queued 2.2 to 2.9 times; a lone CTA is bound by the voxels it takes
+// (512^3 dense prepare 11.8 -> 9.3 ms), a cluster by its rounds, of which bands make more (256^3 dense 2.3 -> 3.4).
+// The band is the largest step wide, so the next band holds the whole list: a distance is at most T plus one
+// step. A soma's seeds lie anywhere: its flood has one band.
 template <int C>
 __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, float *d, int source, int *A, int *B,
-                                float seed_radius = 0.0f) {
+                                int *FA, int *FB, float seed_radius = 0.0f) {
   using G = Group<C>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   if (threadIdx.x == 0) { sh.qn[0] = 0; sh.qn[1] = 0; sh.qn[2] = 0; }
-  if (G::first()) { L->spilled[0] = 0; L->spilled[1] = 0; L->spilled[2] = 0; }
+  if (G::first()) {
+    L->spilled[0] = 0; L->spilled[1] = 0; L->spilled[2] = 0;
+    L->far_n[0] = 0; L->far_n[1] = 0;
+  }
   G::sync();
   uint2 *queue = reinterpret_cast<uint2 *>(queue_bytes());
   int r = -1;  // the seeds are queued for round 0
@@ -411,10 +420,33 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
   const int off = neighbour ? sh.off[lane] : 0;
   const float w = neighbour ? sh.w[lane] : 0.0f;
   const long long bound = capped(a, 8LL * sh.count + 256);
+  const float width = C > 1 || seed_radius > 0.0f ? inf() : a.w[25];
+  float T = width;
+  int p = 0;  // the far list in use
   for (r = 0;; ++r) {
     const Share s = share_of<C>(sh, r % 3, kFloodQueue);
     const int spilled = vload(&L->spilled[r % 3]);
-    if (s.total + spilled == 0) break;
+    if (s.total + spilled == 0) {
+      const int nf = vload(&L->far_n[p]);
+      if (nf == 0) break;
+      if (r >= bound) return false;
+      // the far list becomes round r + 1's frontier (round r's counters may still be read by a CTA that
+      // finds them empty)
+      if (threadIdx.x == 0) sh.qn[(r + 2) % 3] = 0;
+      if (G::first()) L->spilled[(r + 2) % 3] = 0;
+      const int *far = p ? FB : FA;
+      for (int i0 = G::tid() - lane; i0 < nf; i0 += G::threads()) {
+        const int i = i0 + lane;
+        const int v = i < nf ? __ldcg(far + i) : 0;
+        const float dv = i < nf ? __ldcg(d + v) : 0.0f;
+        queue_flood(a, sh, L, i < nf && dv > T, v, __float_as_uint(dv), r, (r & 1) ? A : B);
+      }
+      T = __fadd_rn(T, width);
+      G::sync();
+      if (G::first()) L->far_n[p] = 0;
+      p ^= 1;
+      continue;
+    }
     if (r >= bound) return false;
     if (threadIdx.x == 0) sh.qn[(r + 2) % 3] = 0;
     if (G::first()) L->spilled[(r + 2) % 3] = 0;
@@ -436,22 +468,31 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
         const bool want = neighbour && ((m[j] >> lane) & 1u) && du[j] >= x && cand[j] < dv[j];
         old[j] = want ? atomic_min_pos(d + int(e[j].x) + off, cand[j]) : -1.0f;
       }
-      Places pushed;
+      Places near, later;
 #pragma unroll
-      for (int j = 0; j < kPipe; ++j) pushed.ballot[j] = __ballot_sync(kFull, old[j] > cand[j]);
-      const int n = pushed.total();
-      if (!n) return;
-      const int slot = (r + 1) % 3;
+      for (int j = 0; j < kPipe; ++j) {
+        const bool improved = old[j] > cand[j];
+        near.ballot[j] = __ballot_sync(kFull, improved && cand[j] <= T);
+        later.ballot[j] = __ballot_sync(kFull, improved && cand[j] > T && old[j] == inf());
+      }
+      const int nn = near.total(), nl = later.total();
+      if (!(nn + nl)) return;
+      const int slot = (r + 1) % 3, n = lane == 0 ? nn : lane == 1 ? nl : 0;
       int next = 0;
-      if (lane == 0) next = atomicAdd(&sh.qn[slot], n);
-      pushed.next = __shfl_sync(kFull, next, 0);
+      if (n) next = atomicAdd(lane == 0 ? &sh.qn[slot] : &L->far_n[p], n);
+      near.next = __shfl_sync(kFull, next, 0);
+      later.next = __shfl_sync(kFull, next, 1);
+      int *far = p ? FB : FA;
 #pragma unroll
       for (int j = 0; j < kPipe; ++j) {
         const int v = int(e[j].x) + off;
-        const int q = pushed.take(j);
-        if (!(old[j] > cand[j])) continue;
-        if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
-        else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
+        const int q = near.take(j);
+        if ((near.ballot[j] >> lane) & 1u) {
+          if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
+          else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
+        }
+        const int f = later.take(j);
+        if ((later.ballot[j] >> lane) & 1u) far[f] = v;
       }
     };
     for (int i = s.lo + warp * kPipe; i < s.hi; i += warps * kPipe) {
@@ -512,12 +553,12 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
   Shared *L = G::leader(&sh);
   while (next_object<C>(a, sh, L, big)) {
     const int o = sh.obj;
-    int *A = a.lists + sh.begin, *B = a.lists + a.F + sh.begin;
+    int *A = a.lists + sh.begin, *B = A + a.F, *FA = B + a.F, *FB = FA + a.F;
     int root = a.border_root[o];
     bool ok = true;
     if (root < 0) {
       // the farthest voxel (geometric distance) from the object's first voxel
-      ok = flood_geometric<C>(a, sh, L, a.daf, a.vox[sh.begin], A, B);
+      ok = flood_geometric<C>(a, sh, L, a.daf, a.vox[sh.begin], A, B, FA, FB);
       if (ok) {
         const unsigned long long k = object_argmax<C>(a, sh, L, a.daf);
         root = int(0xFFFFFFFFu - unsigned(k));
@@ -525,7 +566,7 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
         G::sync();
       }
     }
-    if (ok) ok = flood_geometric<C>(a, sh, L, a.daf, root, A, B, a.free_radius[o]);
+    if (ok) ok = flood_geometric<C>(a, sh, L, a.daf, root, A, B, FA, FB, a.free_radius[o]);
     if (!ok) {
       if (G::first()) a.status[o] = kBudget;
       G::sync();
