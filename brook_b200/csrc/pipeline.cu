@@ -709,7 +709,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
     cudaGraph_t graph = nullptr;
     BK_CUDA(cudaStreamEndCapture(s, &graph));
     const auto captured = std::chrono::steady_clock::now();
-    ctx.launch_graph(graph, unsigned(nbig_prepare ? prepare_ctas : 1) | unsigned(nbig_trace ? ctas : 1) << 8);
+    ctx.launch_graph(graph);
     const auto launched = std::chrono::steady_clock::now();
     ctx.stats["host_ms_graph_capture"] = std::chrono::duration<double, std::milli>(captured - graph_start).count();
     ctx.stats["host_ms_graph_launch"] = std::chrono::duration<double, std::milli>(launched - captured).count();

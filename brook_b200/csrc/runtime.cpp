@@ -30,12 +30,7 @@ cudaStream_t Context::copy_stream() {
   return copy_;
 }
 
-void Context::launch_graph(cudaGraph_t graph, unsigned shape) {
-  if (engine_exec_ && engine_shape_ != shape) {
-    cudaGraphExecDestroy(engine_exec_);
-    engine_exec_ = nullptr;
-  }
-  engine_shape_ = shape;
+void Context::launch_graph(cudaGraph_t graph) {
   if (engine_exec_) {
     cudaGraphExecUpdateResultInfo info{};
     if (cudaGraphExecUpdate(engine_exec_, graph, &info) != cudaSuccess) {

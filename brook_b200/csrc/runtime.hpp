@@ -94,9 +94,8 @@ class Context {
   int engine_percent = 100;
   unsigned long long last_class = 0;  // the workload class of the last call
   // Launches a captured graph of the engine's launches: the context keeps one executable graph and
-  // updates it in place when the new graph has the same shape (the caller's number for its kernels and cluster
-  // sizes) and topology; else instantiates it anew.
-  void launch_graph(cudaGraph_t graph, unsigned shape);
+  // updates it in place when the new graph has the same topology (else instantiates it anew).
+  void launch_graph(cudaGraph_t graph);
   // The event a stage mark of a captured graph records: one per stage, kept, since an executable graph
   // whose event nodes change cannot be updated and is instantiated anew (0.3 ms a call).
   cudaEvent_t graph_event(const std::string &stage);
@@ -109,7 +108,6 @@ class Context {
   std::map<void *, size_t> class_of_;           // live and cached blocks -> size class
   size_t cached_ = 0, live_ = 0, peak_ = 0;
   cudaGraphExec_t engine_exec_ = nullptr;
-  unsigned engine_shape_ = 0;
   std::map<std::string, cudaEvent_t> graph_events_;
 };
 
