@@ -54,20 +54,12 @@ void Context::launch_graph(cudaGraph_t graph) {
   stats["graph_launches"] += 1;
 }
 
-cudaEvent_t Context::graph_event(const std::string &stage) {
-  cudaEvent_t &e = graph_events_[stage];
-  if (!e) BK_CUDA(cudaEventCreate(&e));
-  return e;
-}
-
 Context::~Context() {
   if (stream_) {
     int previous = -1;
     cudaGetDevice(&previous);
     cudaSetDevice(device_);
     if (engine_exec_) cudaGraphExecDestroy(engine_exec_);
-    for (auto &entry : graph_events_)
-      if (entry.second) cudaEventDestroy(entry.second);
     if (copy_) {
       cudaStreamSynchronize(copy_);
       cudaStreamDestroy(copy_);

@@ -96,9 +96,6 @@ class Context {
   // Launches a captured graph of the engine's launches: the context keeps one executable graph and
   // updates it in place when the new graph has the same topology (else instantiates it anew).
   void launch_graph(cudaGraph_t graph);
-  // The event a stage mark of a captured graph records: one per stage, kept, since an executable graph
-  // whose event nodes change cannot be updated and is instantiated anew (0.3 ms a call).
-  cudaEvent_t graph_event(const std::string &stage);
 
  private:
   int device_ = 0, sm_count_ = 0;
@@ -108,7 +105,6 @@ class Context {
   std::map<void *, size_t> class_of_;           // live and cached blocks -> size class
   size_t cached_ = 0, live_ = 0, peak_ = 0;
   cudaGraphExec_t engine_exec_ = nullptr;
-  std::map<std::string, cudaEvent_t> graph_events_;
 };
 
 // Device storage that outlives the context that made it (plain cudaMalloc / cudaFree on its
@@ -192,7 +188,6 @@ class Buffer {
 class StageClock {
   Context &ctx_;
   std::vector<std::pair<std::string, cudaEvent_t>> marks_;
-  std::vector<cudaEvent_t> own_;
   std::chrono::steady_clock::time_point host_ = std::chrono::steady_clock::now();
   bool capturing_ = false;
 
@@ -202,18 +197,14 @@ class StageClock {
   // record when the graph runs).
   void capturing(bool on) { capturing_ = on; }
   ~StageClock() {
-    for (cudaEvent_t e : own_) cudaEventDestroy(e);
+    for (auto &m : marks_) cudaEventDestroy(m.second);
   }
   void mark(const std::string &stage) {
     const auto now = std::chrono::steady_clock::now();
     if (!marks_.empty()) ctx_.stats["host_ms_" + stage] += std::chrono::duration<double, std::milli>(now - host_).count();
     host_ = now;
     cudaEvent_t e;
-    if (capturing_) e = ctx_.graph_event(stage);
-    else {
-      BK_CUDA(cudaEventCreate(&e));
-      own_.push_back(e);
-    }
+    BK_CUDA(cudaEventCreate(&e));
     marks_.push_back({stage, e});
     BK_CUDA(cudaEventRecordWithFlags(e, ctx_.stream(), capturing_ ? cudaEventRecordExternal : cudaEventRecordDefault));
   }
