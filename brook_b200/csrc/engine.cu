@@ -647,6 +647,8 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
   const bool neighbour = lane < 26;
   const int off = neighbour ? sh.off[lane] : 0;
   int p = 0;  // the far list in use
+  // The bound counts rounds, which bounds the bands too: after an empty band the nearest deferred offer is the
+  // nearest waiting voxel's own distance, so that voxel is inside the next band.
   const long long bound = capped(a, 16LL * sh.count + 256);
   long long work = 0;
   int r = 0;
@@ -661,10 +663,16 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
       if (least < unsigned(vload(minfar) >> 32) && is && mine == least)
         atomicMin(minfar, (static_cast<unsigned long long>(mine) << 32) | __float_as_uint(penalty));
     };
-    for (;; ++r) {
+    for (const int first_round = r;; ++r) {
       const Share s = share_of<C>(sh, r % 3, kFloodQueue);
       const int spilled = vload(&L->spilled[r % 3]);
-      if (s.total + spilled == 0) break;
+      if (s.total + spilled == 0) {
+        // A band may be empty: the offer that named it can have been improved into the band before it. The
+        // barrier that every round ends with then stands here, between this band's reading of sh.T and the
+        // clearing of the last band's list, before it, and the next band's end and list, after it.
+        if (r == first_round) G::sync();
+        break;
+      }
       if (++work > bound) {
         if (G::first()) L->status = kBudget;
         G::sync();
