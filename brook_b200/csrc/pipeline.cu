@@ -667,8 +667,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   OrderPlan orders = plan_target_orders(ctx, F, nobj, largest, a.delta, a.w[25], wide_order);
   a.order = orders.order.data();
   // the engine's launches, prepare -> target orders -> trace, as one CUDA graph (every buffer is
-  // made above; the graph holds kernels, a memset and the stage marks): one submission per call,
-  // and the context's executable graph is updated in place while the topology holds
+  // made above; the graph holds kernels, a memset and the stage marks): one submission per call
   const char *graph_knob = std::getenv("BROOK_B200_GRAPH");
   const bool as_graph = !fields && !(graph_knob && std::string(graph_knob) == "0");
   auto engine = [&] {

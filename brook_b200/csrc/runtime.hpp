@@ -93,8 +93,9 @@ class Context {
   // take; below 100 another context's kernels find free CTA slots while this one traces.
   int engine_percent = 100;
   unsigned long long last_class = 0;  // the workload class of the last call
-  // Launches a captured graph of the engine's launches: the context keeps one executable graph and
-  // updates it in place when the new graph has the same topology (else instantiates it anew).
+  // Launches a captured graph of the engine's launches, instantiated anew for every call. An executable graph is not
+  // updated in place: calls differ in their kernels and cluster sizes, and whether an update succeeded depended on
+  // the handles that the stage marks' new events happened to get. The context keeps the last one until the next call.
   void launch_graph(cudaGraph_t graph);
 
  private:

@@ -80,9 +80,9 @@ def test_pdrf_exponent_not_a_power_of_two(gpu, monkeypatch, exponent, fix_branch
 
 
 def test_engine_graph_matches_eager_launches(gpu, monkeypatch):
-    """The engine's launches (prepare, target orders, trace) run as one CUDA graph per call; the
-    context updates its executable graph in place for the next call. The skeletons equal those of
-    the same launches made one by one (BROOK_B200_GRAPH=0) and the oracle's."""
+    """The engine's launches (prepare, target orders, trace) run as one CUDA graph, instantiated for
+    each call. The skeletons equal those of the same launches made one by one (BROOK_B200_GRAPH=0)
+    and the oracle's."""
     from brook_b200 import _native, synthetic
 
     labels = synthetic.tube_volume((64, 64, 64), objects=8, seed=9)
@@ -98,6 +98,27 @@ def test_engine_graph_matches_eager_launches(gpu, monkeypatch):
     exp = oracle.skeletonize(labels, threads=8, **opts)
     for got in (first, second, eager):
         assert_same(got, exp, "graph / eager")
+
+
+def test_calls_of_every_cluster_size_in_turn(gpu, monkeypatch):
+    """One context runs engine graphs of lone CTAs, clusters of eight (one object) and clusters of four (seventeen
+    objects of one size, none with the sixteenth of the foreground that calls for eight) in every order; each call
+    launches a graph of its own."""
+    from brook_b200 import _native
+
+    one = np.zeros((24, 22, 21), np.uint8, order="F")
+    one[1:-1, 1:-1, 1:-1] = 1
+    one[8:14, 6:, 5:12] = 0
+    many = np.asfortranarray(np.concatenate([one] * 17, axis=2))
+    opts = dict(teasar_params=dict(CFG0_PARAMS, const=10), anisotropy=(1, 1, 1), dust_threshold=0)
+    expected = [oracle.skeletonize(v, threads=8, **opts) for v in (one, many)]
+    for size in (1, 8, 4, 1, 4, 8, 1):
+        voxels = "100000000" if size == 1 else "1"
+        monkeypatch.setenv("BROOK_B200_PREPARE_CLUSTER_VOXELS", voxels)
+        monkeypatch.setenv("BROOK_B200_TRACE_CLUSTER_VOXELS", voxels)
+        assert_same(bk().skeletonize(many if size == 4 else one, output="packed", **opts), expected[size == 4], str(size))
+        stats = _native.stats()
+        assert stats["graph_instantiations"] == stats["graph_launches"] == 1 and not stats.get("graph_updates")
 
 
 def test_autotune_installs_a_choice_that_keeps_the_skeletons(gpu, monkeypatch, tmp_path):
