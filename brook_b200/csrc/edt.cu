@@ -290,8 +290,11 @@ __global__ void edt_envelope_volumes(const uint32_t *__restrict__ ids, float *__
 // and keeps no stacks in memory (the envelope's: 16 bytes a voxel written and read back). A lane owns
 // a column, so the banks never conflict. The scan is bound by its two shared loads a step; its length is
 // the distance found, a few voxels in segmentations. Past kNearSteps it goes by blocks of 32 voxels,
-// skipping those whose least height cannot improve (0 where a run starts in the block): solid volumes
-// cost n / 32 steps instead of n.
+// skipping those whose least height cannot improve (0 where a run starts in the block, but for the line's first):
+// solid volumes cost n / 32 steps instead of n. A voxel farther from the walls seen so far than the near steps
+// passes over its own block by the same rule, without near steps: with near steps always, thick boxes took longer
+// than with the envelope (a 384^3 box's EDT at (1, 1, 1): envelope 4.9 ms, near steps always 6.8, now 3.0; the three
+// passes of a 512^3 volume without a wall 22.2 -> 4.3, of 512 cells in 320^3 1.45 -> 1.49).
 constexpr int kScanCols = 32, kScanBlock = 32, kNearSteps = 24;
 constexpr unsigned kScanBackground = 0xFFFFFFFFu, kScanStart = 0x80000000u;
 constexpr size_t kScanMaxSmem = 220 * 1024;
@@ -337,22 +340,22 @@ __global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float
   // a warp loads whole blocks of 32 rows, so that a row's previous id is in a register
   for (int b = warp; b < blocks; b += warps) {
     const int p0 = b * kScanBlock, p1 = min(n, p0 + kScanBlock);
-    L before = in && p0 > 0 ? ids[base + (p0 - 1) * stride] : L(0);
+    L before = in ? ids[base + max(p0 - 1, 0) * stride] : L(0);
     float m = __uint_as_float(BK_INF_BITS);
 #pragma unroll 8
     for (int p = p0; p < p1; ++p) {
       const L id = in ? ids[base + p * stride] : L(0);
       const float h = in ? D[base + p * stride] : 0.0f;
-      const bool start = p == 0 || id != before;
+      const bool turn = id != before, start = p == 0 || turn;
       before = id;
-      m = fminf(m, start ? 0.0f : h);
+      m = fminf(m, turn ? 0.0f : h);
       column[p * kScanCols] = id == 0 ? kScanBackground : (__float_as_uint(h) | (start ? kScanStart : 0u));
     }
     least[b * kScanCols] = m;
   }
   __syncthreads();
   if (!in) return;
-  const float w2 = __fmul_rn(v.w, v.w);
+  const float w2 = __fmul_rn(v.w, v.w), distant = __fmul_rn(w2, float(kNearSteps * kNearSteps));
   for (int q = warp; q < n; q += warps) {
     const unsigned own = column[q * kScanCols];
     if (own == kScanBackground) {
@@ -363,8 +366,19 @@ __global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float
     // the low side goes on while the run started below the voxels seen, the high side until a start
     bool low = true, high = true;
     unsigned seen = own;
-    int j = 1;
-    for (; j <= kNearSteps && (low || high); ++j) {
+    int below = 1, above = 0;  // each side's next step
+    if (best > distant) {
+      const int b = q / kScanBlock;
+      if (__fadd_rn(w2, least[b * kScanCols]) >= best) {
+        below = q - b * kScanBlock + 1;
+        seen = b == 0 ? kScanStart : 0u;
+        above = (b + 1) * kScanBlock <= n ? (b + 1) * kScanBlock - q : 1;
+      }
+    }
+    // (above is 0 unless the voxel's own block is passed over)
+    if (!above) for (int j = 1;; ++j) {
+      below = above = j;
+      if (j > kNearSteps || !(low || high)) break;
       const float jj = float(j * j), c = __fmul_rn(w2, jj);
       if (c >= best) { low = high = false; break; }
       if (low) {
@@ -387,7 +401,7 @@ __global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float
       }
     }
     if (low)
-      for (int i = j;; ++i) {
+      for (int i = below;; ++i) {
         const int p = q - i;
         const float ii = float(i * i), c = __fmul_rn(w2, ii);
         if (c >= best) break;
@@ -397,15 +411,15 @@ __global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float
         }
         if ((p & (kScanBlock - 1)) == kScanBlock - 1 &&
             __fmaf_rn(w2, ii, least[p / kScanBlock * kScanCols]) >= best) {
-          i += kScanBlock - 1;  // no start in the block: the run goes on below it
-          seen = 0;
+          i += kScanBlock - 1;  // no start in the block but the line's: the run goes on below it
+          seen = p == kScanBlock - 1 ? kScanStart : 0u;
           continue;
         }
         seen = column[p * kScanCols];
         best = fminf(best, __fmaf_rn(w2, ii, __uint_as_float(seen & ~kScanStart)));
       }
     if (high)
-      for (int i = j;; ++i) {
+      for (int i = above;; ++i) {
         const int p = q + i;
         const float ii = float(i * i), c = __fmul_rn(w2, ii);
         if (c >= best) break;

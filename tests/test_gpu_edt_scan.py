@@ -56,3 +56,17 @@ def test_lines_past_shared_memory(gpu):
     for length in (1677, 1678):
         labels = _labels((7, 2, length), "slabs")
         np.testing.assert_array_equal(_edt(labels, (8, 8, 40), False), oracle.edt(labels, (8, 8, 40), False))
+
+
+@pytest.mark.parametrize("wall", [None, 0, 31, 32, 33, -1])
+@pytest.mark.parametrize("shape", [(97, 64, 65), (130, 95, 34), (64, 63, 160)])
+def test_thick_boxes_match_oracle(gpu, shape, wall):
+    """Voxels farther from the walls than the near steps, whose own block of 32 is passed over: one object with a plane of
+    background across y and z (or none) beside a block's edges, at the line's first and last voxel too."""
+    labels = np.ones(shape, np.uint32, order="F")
+    if wall is not None:
+        labels[:, wall, :] = 0
+        labels[:, :, wall] = 0
+    for aniso in ((1, 1, 1), (4, 3, 2)):
+        for black_border in (False, True):
+            np.testing.assert_array_equal(_edt(labels, aniso, black_border), oracle.edt(labels, aniso, black_border))
