@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(512) edt_scan(const L *__restrict__ ids, float
 // Every height and w2 is 0 or a float32 of at least the least squared spacing, so a whole multiple of
 // that square's last place g; sums stay below V. Numerators and products of the envelope are exact in 53
 // bits below V / g = 2^52, and an intersection lies on a whole voxel or at least g / (2 w2 n) from it,
-// which a division rounding at 2^-53 n resolves below 8 w2 n^2 / g = 2^53. (512 voxels an axis: spacings up
-// to 30 times apart, whatever their own digits.)
+// which a division rounding at 2^-53 n resolves below 8 w2 n^2 / g = 2^53. (512 voxels an axis: spacings up to
+// 11 to 16 times apart, by the least one's digits; 1024: up to 5.6 to 8.)
 bool scan_is_exact(const float *w, const int *n, int axes) {
   double total = 0, last = INFINITY;
   for (int a = 0; a < axes; ++a) {
@@ -456,7 +456,7 @@ bool scan_is_exact(const float *w, const int *n, int axes) {
   return 16.0 * total < last * 9007199254740992.0;
 }
 
-// The line must fit a CTA's shared memory (1677 voxels); longer ones take the envelope.
+// The line must fit a CTA's shared memory (1706 voxels); longer ones take the envelope.
 bool scan_fits(int n) { return scan_smem(n) <= kScanMaxSmem; }
 
 void allow_edt_scan_smem() {

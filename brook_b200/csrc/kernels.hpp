@@ -63,7 +63,8 @@ void edt(Context &ctx, const uint32_t *ids, VolumeDims d, const float aniso[3], 
 void edt_xy_squared(Context &ctx, const uint32_t *ids, VolumeDims d, const float aniso[3], bool black_border, float *D);
 void edt_z_finish(Context &ctx, const uint32_t *ids, VolumeDims d, float wz, bool black_border, float *D);
 // The 3D EDT of integer labels without their components (runs of equal labels along a line are runs of one
-// component); false, with nothing done, where the y and z passes need the envelope.
+// component); false, with nothing done, where the y and z passes need the envelope, the x extent is too long for the x pass
+// or a spacing is not finite and positive.
 bool edt_labels(Context &ctx, const void *labels, int dtype, VolumeDims d, const float aniso[3], bool black_border,
                 float *D);
 struct EdtVolume {

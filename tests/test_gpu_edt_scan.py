@@ -51,11 +51,49 @@ def test_scans_match_oracle(gpu, shape, kind, aniso):
         np.testing.assert_array_equal(_edt(labels, aniso, black_border), oracle.edt(labels, aniso, black_border))
 
 
-def test_lines_past_shared_memory(gpu):
-    """1677 voxels fit a CTA's shared memory, 1678 take the envelope."""
-    for length in (1677, 1678):
-        labels = _labels((7, 2, length), "slabs")
-        np.testing.assert_array_equal(_edt(labels, (8, 8, 40), False), oracle.edt(labels, (8, 8, 40), False))
+@pytest.mark.parametrize("length", [1706, 1707])
+@pytest.mark.parametrize("axis", [1, 2])
+def test_lines_past_shared_memory(gpu, length, axis):
+    """1706 voxels fit a CTA's shared memory, 1707 take the envelope, in that axis's pass alone."""
+    from brook_b200 import _native as n
+    from test_zz_no_alloc import _device_fortran, _edt_noalloc
+    import torch
+
+    labels = _labels((7, length, 3) if axis == 1 else (7, 3, length), "slabs")
+    expected = oracle.edt(labels, (8, 8, 40), False)
+    np.testing.assert_array_equal(_edt(labels, (8, 8, 40), False), expected)
+    out = torch.full((labels.size,), -1.0, dtype=torch.float32, device="cuda")
+    assert _edt_noalloc(_device_fortran(labels.view(np.int32)), out, (8, 8, 40), False,
+                        torch.cuda.current_stream()) == n.SUCCESS
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy().reshape(labels.shape, order="F"), expected)
+
+
+@pytest.mark.parametrize("length", [1706, 1707])
+def test_batch_with_a_long_volume(gpu, length):
+    """The distance fields of a batch, one volume of which has the longest line that scans or one too long for it."""
+    from test_gpu_parity import assert_same, bk
+
+    opts = dict(teasar_params=dict(scale=1.5, const=30, pdrf_scale=100000, pdrf_exponent=4), anisotropy=(8, 8, 40),
+                dust_threshold=10)
+    volumes = [_labels((12, 11, length), "slabs"), _labels((40, 33, 29), "slabs")]
+    got = bk().skeletonize_batch(volumes, output="packed", **opts)
+    for i, v in enumerate(volumes):
+        assert_same(got[i], oracle.skeletonize(v, threads=8, **opts), str(v.shape))
+
+
+def test_envelope_in_batches_of_the_fixed_scratch(gpu):
+    """Spacings that the scans refuse, in a volume whose y pass needs more envelope stacks than the fixed scratch holds."""
+    from brook_b200 import _native as n
+    from test_zz_no_alloc import _device_fortran, _edt_noalloc
+    import torch
+
+    labels, spacing = _labels((256, 256, 64), "slabs"), (0.01, 8, 400)
+    out = torch.full((labels.size,), -1.0, dtype=torch.float32, device="cuda")
+    assert _edt_noalloc(_device_fortran(labels.view(np.int32)), out, spacing, False,
+                        torch.cuda.current_stream()) == n.SUCCESS
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy().reshape(labels.shape, order="F"), oracle.edt(labels, spacing, False))
 
 
 @pytest.mark.parametrize("wall", [None, 0, 31, 32, 33, -1])
