@@ -972,6 +972,10 @@ __device__ __forceinline__ int band_of(unsigned mbits, float delta, int kmin) {
   return k < kmin ? kmin : k;
 }
 
+// The re-claimed voxels of a band that are listed: a sixteenth of the object's voxels. With more, looking at every waiting
+// voxel is the shorter way. (0.3 % on the 512^3 dense workload; up to 11 % in porous objects at spacings 40 times apart.)
+__device__ __forceinline__ int redo_room(const Shared &sh) { return sh.count >> 4; }
+
 // Claim-order invalidation of one path (invalidation_kernels.cuh:105-297; lockstep_coop.inc:530-845):
 // alive path vertices become sources (bottleneck M = 0); a claimed voxel u holding (M, s) offers
 // an alive neighbour v the source s when |aniso (v - s)| < scale DBF[s] + const, with
@@ -1046,7 +1050,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
   };
   auto list_redo = [&](int v) {
     const int at = atomicAdd(&L->n_redo, 1);
-    if (at < sh.count) redo[at] = v;
+    if (at < redo_room(sh)) redo[at] = v;
   };
   const bool neighbour = lane < 26;
   const int off = neighbour ? sh.off[lane] : 0;
@@ -1163,7 +1167,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
     // waiting neighbour of it (the neighbours' keys, then their sources' reach)
     const int nr = vload(&L->n_redo);
     if (nr > 0) {
-      const bool all = nr > sh.count;  // more than the list holds: every waiting voxel
+      const bool all = nr > redo_room(sh);  // more than the list holds: every waiting voxel
       const int m = all ? nf : nr;
       for (int i = G::tid() >> 5; i < m; i += G::threads() >> 5) {
         const int u = __ldcg((all ? far : redo) + i);
