@@ -1,6 +1,7 @@
-"""The objects' voxel lists at the edges of a block's 4096 voxels (volumes of a batch that begin anywhere in one, ids
-that no 16-byte load is aligned to), and target orders among many equal distances with the trimmed distance field
-and, for spacings 1e4 times apart, the whole one. Skeletons must be the oracle's bit for bit."""
+"""The objects' voxel lists of a batch whose volumes begin anywhere in a block of 4096 voxels (the unit by which a voxel's
+volume is looked up), several of them in one block and one over many; and target orders among many equal distances, with
+the sorted bits trimmed to the distances that the spacing allows and, for spacings 1e4 times apart, whole. Skeletons must
+be the oracle's bit for bit."""
 import numpy as np
 import pytest
 
