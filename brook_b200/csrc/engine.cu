@@ -163,9 +163,10 @@ __device__ __forceinline__ long long capped(const EngineArgs &a, long long bound
 // One CTA is resident per SM, so the queues take what leaves L1 its half: 28 KB, which spilled a tenth of the
 // large objects' frontiers to HBM, cost 4 % of the 512^3 dense trace (28.5 -> 27.4 ms) and of an arbor's (37.7 ->
 // 36.1).
-constexpr int kQueueBytes = 96 * 1024;
-constexpr int kFloodQueue = kQueueBytes / 16;         // pairs per buffer
-constexpr int kInvalQueue = kQueueBytes / 56 / 2 * 2;  // pairs per buffer, and records
+// Those of a CTA of W threads, which shares its SM with kEngineThreads / W - 1 others.
+template <int W> constexpr int kQueueBytes = 96 * W;
+template <int W> constexpr int kFloodQueue = kQueueBytes<W> / 16;         // pairs per buffer
+template <int W> constexpr int kInvalQueue = kQueueBytes<W> / 56 / 2 * 2;  // pairs per buffer, and records
 // Frontier voxels a warp has in flight: their loads overlap. Three and four spill registers (512^3 dense trace
 // 27.4, 28.4, 29.9 ms with 2, 3 and 4).
 constexpr int kPipe = 2;
@@ -291,6 +292,7 @@ __device__ __forceinline__ void spill(const EngineArgs &a, int v, unsigned bit, 
 __device__ __forceinline__ unsigned spill_bit(int r) { return (r & 1) ? kSpillOdd : kSpillEven; }
 
 // Queues (v, d) of the lanes with p for round r + 1 of a flood.
+template <int W>
 __device__ __forceinline__ void queue_flood(const EngineArgs &a, Shared &sh, Shared *L, bool p, int v, unsigned d, int r,
                                             int *spill_list) {
   const unsigned b = __ballot_sync(kFull, p);
@@ -298,7 +300,7 @@ __device__ __forceinline__ void queue_flood(const EngineArgs &a, Shared &sh, Sha
   const int slot = (r + 1) % 3;
   const int at = queue_place(sh, p, b, slot);
   if (!p) return;
-  if (at < kFloodQueue) reinterpret_cast<uint2 *>(queue_bytes())[((r + 1) & 1) * kFloodQueue + at] = make_uint2(unsigned(v), d);
+  if (at < kFloodQueue<W>) reinterpret_cast<uint2 *>(queue_bytes())[((r + 1) & 1) * kFloodQueue<W> + at] = make_uint2(unsigned(v), d);
   else spill(a, v, spill_bit(r + 1), spill_list, &L->spilled[slot]);
 }
 
@@ -381,7 +383,7 @@ __device__ float freespace_seed(const EngineArgs &a, int x, int y, int z, int rx
 // (512^3 dense prepare 11.8 -> 9.3 ms), a cluster by its rounds, of which bands make more (256^3 dense 2.3 -> 3.4).
 // The band is the largest step wide, so the next band holds the whole list: a distance is at most T plus one
 // step. A soma's seeds lie anywhere: its flood has one band.
-template <int C>
+template <int C, int W>
 __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, float *d, int source, int *A, int *B,
                                 int *FA, int *FB, float seed_radius = 0.0f) {
   using G = Group<C>;
@@ -408,7 +410,7 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
         s = freespace_seed(a, x, y, z, rx, ry, rz, seed_radius);
         if (s >= 0.0f) d[v] = s;
       }
-      queue_flood(a, sh, L, s >= 0.0f, v, __float_as_uint(s), r, A);
+      queue_flood<W>(a, sh, L, s >= 0.0f, v, __float_as_uint(s), r, A);
     }
   } else if (G::first()) {
     d[source] = 0.0f;
@@ -424,7 +426,7 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
   float T = width;
   int p = 0;  // the far list in use
   for (r = 0;; ++r) {
-    const Share s = share_of<C>(sh, r % 3, kFloodQueue);
+    const Share s = share_of<C>(sh, r % 3, kFloodQueue<W>);
     const int spilled = vload(&L->spilled[r % 3]);
     if (s.total + spilled == 0) {
       const int nf = vload(&L->far_n[p]);
@@ -439,7 +441,7 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
         const int i = i0 + lane;
         const int v = i < nf ? __ldcg(far + i) : 0;
         const float dv = i < nf ? __ldcg(d + v) : 0.0f;
-        queue_flood(a, sh, L, i < nf && dv > T, v, __float_as_uint(dv), r, (r & 1) ? A : B);
+        queue_flood<W>(a, sh, L, i < nf && dv > T, v, __float_as_uint(dv), r, (r & 1) ? A : B);
       }
       T = __fadd_rn(T, width);
       G::sync();
@@ -488,7 +490,7 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
         const int v = int(e[j].x) + off;
         const int q = near.take(j);
         if ((near.ballot[j] >> lane) & 1u) {
-          if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
+          if (q < kFloodQueue<W>) queue[((r + 1) & 1) * kFloodQueue<W> + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
           else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
         }
         const int f = later.take(j);
@@ -501,7 +503,7 @@ __device__ bool flood_geometric(const EngineArgs &a, Shared &sh, Shared *L, floa
       for (int j = 0; j < kPipe; ++j) {
         int q, at;
         locate<C>(s, min(i + j, s.hi - 1), q, at);
-        e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue + at];
+        e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue<W> + at];
         if (i + j >= s.hi) e[j].y = BK_INF_BITS;  // past the share: relaxes nothing
       }
       relax(e);
@@ -546,7 +548,7 @@ __device__ unsigned long long object_argmax(const EngineArgs &a, Shared &sh, Sha
   return r;
 }
 
-template <int C>
+template <int C, int W>
 __device__ void prepare_loop(const EngineArgs &a, bool big) {
   using G = Group<C>;
   __shared__ Shared sh;
@@ -558,7 +560,7 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
     bool ok = true;
     if (root < 0) {
       // the farthest voxel (geometric distance) from the object's first voxel
-      ok = flood_geometric<C>(a, sh, L, a.daf, a.vox[sh.begin], A, B, FA, FB);
+      ok = flood_geometric<C, W>(a, sh, L, a.daf, a.vox[sh.begin], A, B, FA, FB);
       if (ok) {
         const unsigned long long k = object_argmax<C>(a, sh, L, a.daf);
         root = int(0xFFFFFFFFu - unsigned(k));
@@ -566,7 +568,7 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
         G::sync();
       }
     }
-    if (ok) ok = flood_geometric<C>(a, sh, L, a.daf, root, A, B, FA, FB, a.free_radius[o]);
+    if (ok) ok = flood_geometric<C, W>(a, sh, L, a.daf, root, A, B, FA, FB, a.free_radius[o]);
     if (!ok) {
       if (G::first()) a.status[o] = kBudget;
       G::sync();
@@ -600,10 +602,10 @@ __device__ void prepare_loop(const EngineArgs &a, bool big) {
 // CTA takes small objects on its own: large objects start first (they set the kernel's length),
 // and no CTA idles while any object is left.
 // (C == 1: a launch without large objects.)
-template <int C>
-__global__ void __launch_bounds__(kEngineThreads, 1) prepare_kernel(const __grid_constant__ EngineArgs a) {
-  if constexpr (C > 1) prepare_loop<C>(a, true);
-  prepare_loop<1>(a, false);
+template <int C, int W>
+__global__ void __launch_bounds__(W, kEngineThreads / W) prepare_kernel(const __grid_constant__ EngineArgs a) {
+  if constexpr (C > 1) prepare_loop<C, W>(a, true);
+  prepare_loop<1, W>(a, false);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1) prepare_kernel(const __grid
 // nearest rail's) is exact when the flood stops.
 // The far list holds the voxels first reached beyond T (at their first touch, so once each); one
 // whose distance is at most the T before has since been queued as near.
-template <int C>
+template <int C, int W>
 __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *L, int t, int *A, int *B, int *FA,
                                        int *FB, int *touched) {
   using G = Group<C>;
@@ -664,7 +666,7 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
         atomicMin(minfar, (static_cast<unsigned long long>(mine) << 32) | __float_as_uint(penalty));
     };
     for (const int first_round = r;; ++r) {
-      const Share s = share_of<C>(sh, r % 3, kFloodQueue);
+      const Share s = share_of<C>(sh, r % 3, kFloodQueue<W>);
       const int spilled = vload(&L->spilled[r % 3]);
       if (s.total + spilled == 0) {
         // A band may be empty: the offer that named it can have been improved into the band before it. The
@@ -726,7 +728,7 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
           const int v = int(e[j].x) + off;
           const int q = near.take(j);
           if ((near.ballot[j] >> lane) & 1u) {
-            if (q < kFloodQueue) queue[((r + 1) & 1) * kFloodQueue + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
+            if (q < kFloodQueue<W>) queue[((r + 1) & 1) * kFloodQueue<W> + q] = make_uint2(unsigned(v), __float_as_uint(cand[j]));
             else spill(a, v, spill_bit(r + 1), nxt, &L->spilled[slot]);
           }
           const int w = first.take(j);
@@ -748,7 +750,7 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
         for (int j = 0; j < kPipe; ++j) {
           int q, at;
           locate<C>(s, min(i + j, s.hi - 1), q, at);
-          e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue + at];
+          e[j] = of_rank<C>(queue, q)[(r & 1) * kFloodQueue<W> + at];
           if (i + j >= s.hi) e[j].y = BK_INF_BITS;  // past the share: relaxes nothing
         }
         relax(e);
@@ -818,7 +820,7 @@ __device__ unsigned long long railroad(const EngineArgs &a, Shared &sh, Shared *
         fw = a.pdrf[w];
       }
       const bool waits = i < nf && dw > T;
-      queue_flood(a, sh, L, waits && dw <= Tn, w, __float_as_uint(dw), r, nxt);
+      queue_flood<W>(a, sh, L, waits && dw <= Tn, w, __float_as_uint(dw), r, nxt);
       append(waits && dw > Tn, w, keep, &L->far_n[p ^ 1]);
       defer(waits && dw > Tn, dw, fw);
     }
@@ -998,15 +1000,15 @@ __device__ __forceinline__ int redo_room(const Shared &sh) { return sh.count >> 
 // key, position relative to the source and the source's reach. Step B makes the offers, a warp per
 // voxel: one L2 read per neighbour decides it (dead, holding a better key or offer, or out of reach:
 // done), an atomic follows only where the key changes.
-template <int C>
+template <int C, int W>
 __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int *path, int npath, int *A, int *B,
                            int *FA, int *FB, int *touched, int *redo, unsigned long long *wide) {
   using G = Group<C>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   int4 *stage_id = reinterpret_cast<int4 *>(queue_bytes());           // voxel, mask, source + 1, M bits
-  float4 *stage_at = reinterpret_cast<float4 *>(stage_id + kInvalQueue);  // position - source's, reach
-  unsigned long long *queue_key = reinterpret_cast<unsigned long long *>(stage_at + kInvalQueue);
-  int *queue_vox = reinterpret_cast<int *>(queue_key + 2 * kInvalQueue);
+  float4 *stage_at = reinterpret_cast<float4 *>(stage_id + kInvalQueue<W>);  // position - source's, reach
+  unsigned long long *queue_key = reinterpret_cast<unsigned long long *>(stage_at + kInvalQueue<W>);
+  int *queue_vox = reinterpret_cast<int *>(queue_key + 2 * kInvalQueue<W>);
   if (threadIdx.x == 0) {
     sh.qn[0] = 0; sh.qn[1] = 0; sh.qn[2] = 0;
     sh.lowest[0] = BK_INF_BITS; sh.lowest[1] = BK_INF_BITS;
@@ -1024,9 +1026,9 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
     if (!b) return;
     const int at = queue_place(sh, p, b, slot);
     if (!p) return;
-    if (at < kInvalQueue) {
-      queue_vox[buffer * kInvalQueue + at] = v;
-      queue_key[buffer * kInvalQueue + at] = k;
+    if (at < kInvalQueue<W>) {
+      queue_vox[buffer * kInvalQueue<W> + at] = v;
+      queue_key[buffer * kInvalQueue<W> + at] = k;
     } else spill(a, v, kFront, spill_list, &L->spilled[slot]);
   };
   for (int i0 = G::tid() - lane; i0 < npath; i0 += G::threads()) {
@@ -1064,7 +1066,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
     int *far = p ? FB : FA, *keep = p ? FA : FB;
     unsigned hi = __float_as_uint(__fmul_rn(float(band + 1), a.delta));
     for (;; ++r) {
-      const Share s = share_of<C>(sh, r % 3, kInvalQueue);
+      const Share s = share_of<C>(sh, r % 3, kInvalQueue<W>);
       const int spilled = vload(&L->spilled[r % 3]);
       if (s.total + spilled == 0) break;
       if (++work > bound) return false;
@@ -1077,8 +1079,8 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
         int q, at;
         locate<C>(s, min(i, s.hi - 1), q, at);
         if (i < s.hi) {
-          const int u = of_rank<C>(queue_vox, q)[(r & 1) * kInvalQueue + at];
-          const unsigned long long k = of_rank<C>(queue_key, q)[(r & 1) * kInvalQueue + at];
+          const int u = of_rank<C>(queue_vox, q)[(r & 1) * kInvalQueue<W> + at];
+          const unsigned long long k = of_rank<C>(queue_key, q)[(r & 1) * kInvalQueue<W> + at];
           const unsigned m = a.mask[u];
           const bool current = __ldcg(a.key + u) == k;
           stage(i - s.lo, u, current ? int(m) : 0, k);
@@ -1092,7 +1094,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
       G::sync();
       // step B: a warp per voxel; the spilled voxels come after the queued ones, staged by this CTA
       int staged = s.hi - s.lo;
-      for (int base = G::rank() * kInvalQueue;;) {
+      for (int base = G::rank() * kInvalQueue<W>;;) {
         for (int i = warp * kPipe; i < staged; i += warps * kPipe) {
           unsigned long long kv[kPipe], old[kPipe];
           unsigned hb[kPipe];  // the offers' upper words
@@ -1128,7 +1130,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
             if (claims && old[j] < kWaits) list_redo(e.x + off);
           }
           if (!any) continue;
-          const int slot = (r + 1) % 3, buffer = ((r + 1) & 1) * kInvalQueue;
+          const int slot = (r + 1) % 3, buffer = ((r + 1) & 1) * kInvalQueue<W>;
           reserve(claimed, first, waits, &sh.qn[slot], &L->n_touch, &L->far_n[p]);
 #pragma unroll
           for (int j = 0; j < kPipe; ++j) {
@@ -1136,7 +1138,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
             const int v = e.x + off;
             const int q = claimed.take(j);
             if ((claimed.ballot[j] >> lane) & 1u) {
-              if (q < kInvalQueue) {
+              if (q < kInvalQueue<W>) {
                 queue_vox[buffer + q] = v;
                 queue_key[buffer + q] = (static_cast<unsigned long long>(hb[j]) << 32) | unsigned(e.z);
               } else spill(a, v, kFront, nxt, &L->spilled[slot]);
@@ -1149,13 +1151,13 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
         }
         if (base >= spilled) break;
         __syncthreads();  // the records are free
-        staged = min(kInvalQueue, spilled - base);
+        staged = min(kInvalQueue<W>, spilled - base);
         for (int i = threadIdx.x; i < staged; i += blockDim.x) {
           const int u = __ldcg(cur + base + i);
           const unsigned long long k = __ldcg(wide + base + i);
           stage(i, u, int(a.mask[u]), k);
         }
-        base += C * kInvalQueue;
+        base += C * kInvalQueue<W>;
         __syncthreads();
       }
       G::sync();
@@ -1255,7 +1257,7 @@ __device__ bool invalidate(const EngineArgs &a, Shared &sh, Shared *L, const int
 
 // A function of its own: inlined into a kernel of lone CTAs the same loop took 33.1 ms of the 512^3 dense
 // trace and 23.3 as a call, on the same 148 CTAs (64 registers either way).
-template <int C>
+template <int C, int W>
 __device__ __noinline__ void trace_loop(const EngineArgs &a, bool big) {
   using G = Group<C>;
   __shared__ Shared sh;
@@ -1339,7 +1341,7 @@ __device__ __noinline__ void trace_loop(const EngineArgs &a, bool big) {
         if (G::first()) store[used] = sh.root;  // the ball's one source (the slot is reused)
         G::sync();
       } else if (step == 1 || a.fix_branching) {
-        const unsigned long long rb = railroad<C>(a, sh, L, step == 1 ? sh.root : t, L0, L1, L2, L3, L4);
+        const unsigned long long rb = railroad<C, W>(a, sh, L, step == 1 ? sh.root : t, L0, L1, L2, L3, L4);
         lap(1);
         if (vload(&L->status) != kOk) { status = vload(&L->status); break; }
         const int nt = vload(&L->n_touch);
@@ -1407,7 +1409,7 @@ __device__ __noinline__ void trace_loop(const EngineArgs &a, bool big) {
         sh.rconst = ball ? a.soma_constant : a.constant;
       }
       __syncthreads();
-      if (!invalidate<C>(a, sh, L, store + used, len, L0, L1, L2, L3, L4, L5, wide)) {
+      if (!invalidate<C, W>(a, sh, L, store + used, len, L0, L1, L2, L3, L4, L5, wide)) {
         status = kBudget;
         break;
       }
@@ -1451,26 +1453,33 @@ __device__ __noinline__ void trace_loop(const EngineArgs &a, bool big) {
 // then join the large ones; the others take the large objects first. So the longest lone-CTA
 // objects run beside the clusters' objects from the start instead of after them. (C == 1: a launch
 // without large objects.)
-template <int C>
-__global__ void __launch_bounds__(kEngineThreads, 1) trace_kernel(const __grid_constant__ EngineArgs a) {
-  if constexpr (C == 1) trace_loop<1>(a, false);
+template <int C, int W>
+__global__ void __launch_bounds__(W, kEngineThreads / W) trace_kernel(const __grid_constant__ EngineArgs a) {
+  if constexpr (C == 1) trace_loop<1, W>(a, false);
   else if (int(blockIdx.x) / C < a.lone_first) {
-    trace_loop<1>(a, false);
-    trace_loop<C>(a, true);
+    trace_loop<1, W>(a, false);
+    trace_loop<C, W>(a, true);
   } else {
-    trace_loop<C>(a, true);
-    trace_loop<1>(a, false);
+    trace_loop<C, W>(a, true);
+    trace_loop<1, W>(a, false);
   }
 }
 
-cudaLaunchConfig_t cluster_config(int clusters, int ctas, cudaStream_t stream, cudaLaunchAttribute *attr) {
+// A kernel, its CTAs' number in a cluster and threads.
+struct Variant {
+  const void *kernel;
+  int ctas, threads;
+  int queue_bytes() const { return kQueueBytes<1> * threads; }
+};
+
+cudaLaunchConfig_t cluster_config(int clusters, const Variant &k, cudaStream_t stream, cudaLaunchAttribute *attr) {
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(unsigned(clusters * ctas));
-  config.blockDim = dim3(kEngineThreads);
-  config.dynamicSmemBytes = kQueueBytes;
+  config.gridDim = dim3(unsigned(clusters * k.ctas));
+  config.blockDim = dim3(unsigned(k.threads));
+  config.dynamicSmemBytes = size_t(k.queue_bytes());
   config.stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(ctas);
+  attr[0].val.clusterDim.x = unsigned(k.ctas);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   config.attrs = attr;
@@ -1478,38 +1487,53 @@ cudaLaunchConfig_t cluster_config(int clusters, int ctas, cudaStream_t stream, c
   return config;
 }
 
-// Resident clusters of `kernel` on the current device (queried once per device and kernel: the
+// Resident clusters of a kernel on the current device (queried once per device and kernel: the
 // query costs far more than a launch).
-int resident_clusters(const void *kernel, int ctas, cudaStream_t stream) {
+int resident_clusters(const Variant &k, cudaStream_t stream) {
   static std::mutex lock;
   static std::map<std::pair<int, const void *>, int> known;
   int device = 0;
   BK_CUDA(cudaGetDevice(&device));
   std::lock_guard<std::mutex> guard(lock);
-  auto it = known.find({device, kernel});
+  auto it = known.find({device, k.kernel});
   if (it != known.end()) return it->second;
   // once per device and kernel, before its first launch
-  BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQueueBytes));
+  BK_CUDA(cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.queue_bytes()));
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t probe = cluster_config(1, ctas, stream, attr);
+  cudaLaunchConfig_t probe = cluster_config(1, k, stream, attr);
   int cap = 1;
-  BK_CUDA(cudaOccupancyMaxActiveClusters(&cap, kernel, &probe));
-  known[{device, kernel}] = cap;
+  BK_CUDA(cudaOccupancyMaxActiveClusters(&cap, k.kernel, &probe));
+  known[{device, k.kernel}] = cap;
   return cap;
 }
 
 // As many clusters as are resident at once (no more than the work needs).
-void launch(const void *kernel, int ctas, const EngineArgs &a, int nbig, cudaStream_t stream, int lone_percent = 0) {
+void launch(const Variant &k, const EngineArgs &a, int nbig, cudaStream_t stream, int lone_percent = 0) {
   EngineArgs args = a;
   args.nbig = nbig;
   void *kargs[] = {&args};
   cudaLaunchAttribute attr[1];
-  const int cap = std::max(1, resident_clusters(kernel, ctas, stream) * std::min(100, std::max(1, a.grid_percent)) / 100);
-  const long long need = nbig + (a.nobj - nbig + ctas - 1) / ctas;
+  const int cap = std::max(1, resident_clusters(k, stream) * std::min(100, std::max(1, a.grid_percent)) / 100);
+  const long long need = nbig + (a.nobj - nbig + k.ctas - 1) / k.ctas;
   const int clusters = int(std::max(1LL, std::min<long long>(cap, need)));
   args.lone_first = nbig > 0 && nbig < a.nobj ? clusters * lone_percent / 100 : 0;
-  cudaLaunchConfig_t config = cluster_config(clusters, ctas, stream, attr);
-  BK_CUDA(cudaLaunchKernelExC(&config, kernel, kargs));
+  cudaLaunchConfig_t config = cluster_config(clusters, k, stream, attr);
+  BK_CUDA(cudaLaunchKernelExC(&config, k.kernel, kargs));
+}
+
+// The tiny objects in a launch of their own after the others'.
+int launch_all(const Variant &k, const Variant &tiny, const EngineArgs &a, int nbig, cudaStream_t stream,
+               int lone_percent = 0) {
+  EngineArgs part = a;
+  part.nobj = a.nobj - a.ntiny;
+  if (part.nobj > 0) launch(k, part, nbig, stream, lone_percent);
+  if (a.ntiny == 0) return 1;
+  const int rest = part.nobj;
+  part.nobj = a.ntiny;
+  part.schedule = a.schedule + rest;
+  part.queue = a.queue + 1;
+  launch(tiny, part, 0, stream);
+  return rest > 0 ? 2 : 1;
 }
 
 }  // namespace
@@ -1525,8 +1549,10 @@ static long long resident_ctas() {
   if (it == known.end()) {
     int sms = 1, per_sm = 1;
     BK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    BK_CUDA(cudaFuncSetAttribute(trace_kernel<kClusterCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQueueBytes));
-    BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas>, kEngineThreads, kQueueBytes));
+    BK_CUDA(cudaFuncSetAttribute(trace_kernel<kClusterCtas, kEngineThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kQueueBytes<kEngineThreads>));
+    BK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kClusterCtas, kEngineThreads>,
+                                                          kEngineThreads, kQueueBytes<kEngineThreads>));
     it = known.emplace(device, std::max(1LL, (long long)sms * per_sm)).first;
   }
   return it->second;
@@ -1547,33 +1573,36 @@ int cluster_ctas(long long largest, long long foreground) {
 
 // The kernel for nbig large objects. Without any, CTAs are launched alone: clusters of 4 fit only 132 of the 148
 // SMs, since an SM short of a whole cluster in its part of the chip stays idle.
-static const void *prepare_variant(int nbig, int &ctas) {
-  if (nbig == 0) { ctas = 1; return (const void *)prepare_kernel<1>; }
-  if (ctas == kWideClusterCtas) return (const void *)prepare_kernel<kWideClusterCtas>;
-  ctas = kClusterCtas;
-  return (const void *)prepare_kernel<kClusterCtas>;
+static Variant prepare_variant(int nbig, int ctas) {
+  if (nbig == 0) return {(const void *)prepare_kernel<1, kEngineThreads>, 1, kEngineThreads};
+  if (ctas == kWideClusterCtas)
+    return {(const void *)prepare_kernel<kWideClusterCtas, kEngineThreads>, kWideClusterCtas, kEngineThreads};
+  return {(const void *)prepare_kernel<kClusterCtas, kEngineThreads>, kClusterCtas, kEngineThreads};
 }
-static const void *trace_variant(int nbig, int &ctas) {
-  if (nbig == 0) { ctas = 1; return (const void *)trace_kernel<1>; }
-  if (ctas == kWideClusterCtas) return (const void *)trace_kernel<kWideClusterCtas>;
-  ctas = kClusterCtas;
-  return (const void *)trace_kernel<kClusterCtas>;
+static Variant trace_variant(int nbig, int ctas) {
+  if (nbig == 0) return {(const void *)trace_kernel<1, kEngineThreads>, 1, kEngineThreads};
+  if (ctas == kWideClusterCtas)
+    return {(const void *)trace_kernel<kWideClusterCtas, kEngineThreads>, kWideClusterCtas, kEngineThreads};
+  return {(const void *)trace_kernel<kClusterCtas, kEngineThreads>, kClusterCtas, kEngineThreads};
+}
+static Variant tiny_prepare() { return {(const void *)prepare_kernel<1, kTinyThreads>, 1, kTinyThreads}; }
+static Variant tiny_trace() { return {(const void *)trace_kernel<1, kTinyThreads>, 1, kTinyThreads}; }
+
+int launch_prepare(const EngineArgs &a, int nbig, int ctas, cudaStream_t stream) {
+  return launch_all(prepare_variant(nbig, ctas), tiny_prepare(), a, nbig, stream);
 }
 
-void launch_prepare(const EngineArgs &a, int nbig, int ctas, cudaStream_t stream) {
-  const void *kernel = prepare_variant(nbig, ctas);
-  launch(kernel, ctas, a, nbig, stream);
+void prepare_engine_launches(int ntiny, int nbig_prepare, int prepare_ctas, int nbig_trace, int trace_ctas,
+                             cudaStream_t stream) {
+  resident_clusters(prepare_variant(nbig_prepare, prepare_ctas), stream);
+  resident_clusters(trace_variant(nbig_trace, trace_ctas), stream);
+  if (ntiny == 0) return;
+  resident_clusters(tiny_prepare(), stream);
+  resident_clusters(tiny_trace(), stream);
 }
 
-void prepare_engine_launches(int nbig_prepare, int prepare_ctas, int nbig_trace, int trace_ctas, cudaStream_t stream) {
-  const void *prepare = prepare_variant(nbig_prepare, prepare_ctas), *trace = trace_variant(nbig_trace, trace_ctas);
-  resident_clusters(prepare, prepare_ctas, stream);
-  resident_clusters(trace, trace_ctas, stream);
-}
-
-void launch_trace(const EngineArgs &a, int nbig, int ctas, int lone_percent, cudaStream_t stream) {
-  const void *kernel = trace_variant(nbig, ctas);
-  launch(kernel, ctas, a, nbig, stream, lone_percent);
+int launch_trace(const EngineArgs &a, int nbig, int ctas, int lone_percent, cudaStream_t stream) {
+  return launch_all(trace_variant(nbig, ctas), tiny_trace(), a, nbig, stream, lone_percent);
 }
 
 }  // namespace bk

@@ -11,7 +11,7 @@
 
 namespace bk {
 
-// Threads per CTA: one CTA per SM at the 64 registers its floods need without spills. A frontier
+// Threads per CTA: one CTA per SM at 64 registers (the trace's loop spills some 70 words of state). A frontier
 // voxel is a warp's work, so an object's rounds are as fast as its warps are many, and a lone CTA's
 // barrier costs a fraction of a cluster's. On the 512^3 dense workload (trace ms, every object on one
 // CTA) 256 threads 57.7, 512 35.7, 1024 29.7.
@@ -53,7 +53,8 @@ struct EngineArgs {
   const int *schedule;   // processing order (object indices): large objects first, then the rest
   int nbig;              // schedule[0, nbig) run on clusters (set by launch_prepare / launch_trace)
   int lone_first;        // trace: clusters [0, lone_first) take the small objects first
-  int *queue;            // two work counters (large, small), both 0 at launch
+  int ntiny;             // the schedule's last ntiny objects take a launch of small CTAs after the others'
+  int *queue;            // three work counters (large, small, tiny), 0 at launch
   int *status;           // per object
   int *lists;            // 6 lists of F ints: list w of object o at lists + w * F + obj_begin[o]
   unsigned long long *wide;  // F entries: object o at wide + obj_begin[o] (a spilled frontier's keys)
@@ -134,11 +135,20 @@ long long trace_cluster_voxels(long long foreground);
 constexpr long long kPrepareClusterFloor = 4096, kPrepareWholeShare = 32768;
 long long prepare_cluster_voxels(long long foreground);
 
+// Tiny objects, below kTinyVoxels, take small CTAs, four to an SM, when a call has at least kTinyObjects of them: their
+// chains are a few dozen rounds of barriers and L2 round trips, which a CTA that fills an SM serves one object at a time.
+// They are launched after the others', in whose shadow a few of them cost nothing. Measured (prepare + trace ms, all on
+// large CTAs and with small ones of 256 threads; of 128): 32768 cubes of 6^3 26.5, 8.7, 6.1; 15625 of 8^3 19.5, 7.9, 6.5;
+// 4096 of 13^3 11.7, 6.7, 6.4; 2744 of 16^3 13.2, 9.4, 10.2; 1331 of 20^3 10.3, 9.1, 11.1; 2048 of 6^3 1.5, 0.6, 0.4.
+constexpr int kTinyThreads = 256;
+constexpr int kTinyVoxels = 4096, kTinyObjects = 1024;
+
 // One pass of the engine: clusters take schedule[0, nbig) (large objects, largest first), then
-// every CTA takes schedule[nbig, nobj) alone. queue[0] and queue[1] must be zero.
-void launch_prepare(const EngineArgs &a, int nbig, int cluster_ctas, cudaStream_t stream);
+// every CTA takes schedule[nbig, nobj - ntiny) alone, then small CTAs the rest. The queue's counters must be zero.
+// Returns the launches made.
+int launch_prepare(const EngineArgs &a, int nbig, int cluster_ctas, cudaStream_t stream);
 // lone_percent: the share of clusters (percent) whose CTAs take small objects first.
-void launch_trace(const EngineArgs &a, int nbig, int cluster_ctas, int lone_percent, cudaStream_t stream);
+int launch_trace(const EngineArgs &a, int nbig, int cluster_ctas, int lone_percent, cudaStream_t stream);
 constexpr int kLoneFirstPercent = 10;
 // The railroad band's width in penalties of the nearest deferred voxel (EngineArgs::rail_band).
 // Measured on the 512^3 dense workload (trace ms): 0.1 69.8, 0.25 59.0, 0.5 56.1, 1 58.4, 2 60.6,
@@ -146,7 +156,7 @@ constexpr int kLoneFirstPercent = 10;
 constexpr float kRailBand = 0.5f;
 // The device queries the launches above make (resident clusters per kernel), done ahead so that
 // a stream capture of the launches holds launches only.
-void prepare_engine_launches(int nbig_prepare, int prepare_cluster_ctas, int nbig_trace, int trace_cluster_ctas,
-                             cudaStream_t stream);
+void prepare_engine_launches(int ntiny, int nbig_prepare, int prepare_cluster_ctas, int nbig_trace,
+                             int trace_cluster_ctas, cudaStream_t stream);
 
 }  // namespace bk

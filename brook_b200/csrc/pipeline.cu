@@ -595,6 +595,9 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
                                    tune.prepare_cluster_voxels > 0 ? tune.prepare_cluster_voxels : prepare_cluster_voxels(F));
   const int nbig_trace = leading("BROOK_B200_TRACE_CLUSTER_VOXELS",
                                  tune.trace_cluster_voxels > 0 ? tune.trace_cluster_voxels : trace_cluster_voxels(F));
+  int ntiny = 0;
+  while (ntiny < nobj - std::max(nbig_prepare, nbig_trace) && obj_count[schedule[nobj - 1 - ntiny]] < kTinyVoxels) ++ntiny;
+  if (ntiny < kTinyObjects) ntiny = 0;
   auto d_arena_offset = to_device(ctx, arena_offset), d_arena_dims = to_device(ctx, arena_dims);
   auto d_obj_arena = to_device(ctx, obj_arena), d_obj_begin = to_device(ctx, obj_begin), d_obj_count = to_device(ctx, obj_count);
   auto d_schedule = to_device(ctx, schedule), d_border_root = to_device(ctx, border_root);
@@ -606,7 +609,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   auto d_after = to_device(ctx, after.empty() ? std::vector<int>{0} : after);
   auto d_max_paths = to_device(ctx, max_paths), d_store_begin = to_device(ctx, store_begin), d_store_cap = to_device(ctx, store_cap);
   auto d_rec_begin = to_device(ctx, rec_begin), d_rec_cap = to_device(ctx, rec_cap);
-  Buffer<int> queue(ctx, 2), status(ctx, nobj), root(ctx, nobj), target(ctx, nobj), npaths(ctx, nobj), nstore(ctx, nobj);
+  Buffer<int> queue(ctx, 3), status(ctx, nobj), root(ctx, nobj), target(ctx, nobj), npaths(ctx, nobj), nstore(ctx, nobj);
   Buffer<float> max_daf(ctx, nobj);
   Buffer<int> lists(ctx, 6 * F), store(ctx, store_total), rec_start(ctx, rec_total), rec_len(ctx, rec_total);
   Buffer<unsigned long long> wide(ctx, F), work(ctx, 4), profile(ctx, 8LL * nobj);
@@ -619,7 +622,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   a.mask = mask.data(); a.dbf = dbf.data(); a.pdrf = pdrf.data(); a.dist = dist.data(); a.daf = daf.data();
   a.flags = flags.data(); a.key = key.data(); a.n = unsigned(NT);
   a.nobj = nobj; a.obj_begin = d_obj_begin.data(); a.obj_count = d_obj_count.data(); a.vox = vox.data();
-  a.schedule = d_schedule.data(); a.queue = queue.data(); a.status = status.data();
+  a.schedule = d_schedule.data(); a.ntiny = ntiny; a.queue = queue.data(); a.status = status.data();
   a.lists = lists.data(); a.wide = wide.data(); a.F = F;
   a.border_root = d_border_root.data(); a.M = d_M.data(); a.pdrf_scale = float(t.pdrf_scale); a.squarings = squarings;
   a.exponent = float(exponent);
@@ -671,8 +674,7 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   const char *graph_knob = std::getenv("BROOK_B200_GRAPH");
   const bool as_graph = !fields && !(graph_knob && std::string(graph_knob) == "0");
   auto engine = [&] {
-    launch_prepare(a, nbig_prepare, prepare_ctas, s);
-    ++ctx.launches;
+    ctx.launches += launch_prepare(a, nbig_prepare, prepare_ctas, s);
     clock.mark("prepare");
     if (fields) {
       // diagnostics: the prepared DAF and PDRF (root rails included) as raw float32 files
@@ -683,15 +685,14 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
       }
     }
     run_target_orders(ctx, orders, vox.data(), daf.data(), d_obj_begin.data());
-    BK_CUDA(cudaMemsetAsync(queue.data(), 0, 2 * sizeof(int), s));
+    BK_CUDA(cudaMemsetAsync(queue.data(), 0, 3 * sizeof(int), s));
     clock.mark("order");
-    launch_trace(a, nbig_trace, ctas, lone_percent, s);
-    ++ctx.launches;
+    ctx.launches += launch_trace(a, nbig_trace, ctas, lone_percent, s);
     clock.mark("trace");
   };
   if (as_graph) {
     const auto graph_start = std::chrono::steady_clock::now();
-    prepare_engine_launches(nbig_prepare, prepare_ctas, nbig_trace, ctas, s);  // device queries, before the capture
+    prepare_engine_launches(a.ntiny, nbig_prepare, prepare_ctas, nbig_trace, ctas, s);  // device queries, before the capture
     BK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     clock.capturing(true);
     try {
