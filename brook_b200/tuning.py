@@ -3,7 +3,8 @@ caller's own volumes (the C ABI's brook_autotune: a coordinate search over the c
 cluster thresholds and the lone-first share, the engine's device time per candidate), installs the
 fastest for the volumes' workload class in the calling thread's context, and saves it in a JSON
 table keyed by GPU name and workload class. Every context made later loads the table's entries for
-its GPU, so a tuned class stays tuned across processes.
+its GPU, so a tuned class stays tuned across processes. Entries name the engine they were measured on;
+those of another engine are left out, since its choices would stand against this engine's own rules.
 
 The table lives at $BROOK_B200_TUNING_CACHE, else ~/.cache/brook_b200/tuning.json."""
 from __future__ import annotations
@@ -18,6 +19,7 @@ import numpy as np
 from . import _native
 
 _lock = threading.Lock()
+ENGINE = 2  # raised with a change of the engine that its launch choices depend on
 FIELDS = ("trace_cluster_ctas", "trace_cluster_voxels", "prepare_cluster_voxels", "lone_first_percent")
 
 
@@ -44,9 +46,11 @@ def _read():
 
 
 def install_saved(context, device):
-    """Installs the saved choices for this GPU into a new context (nothing when there are none)."""
+    """Installs the choices saved for this GPU and engine into a new context (nothing when there are none)."""
     table = _read().get(_gpu_name(device), {})
     for key, entry in table.items():
+        if entry.get("engine", 1) != ENGINE:
+            continue
         t = _native.Tuning(*(int(entry[f]) for f in FIELDS))
         _native.check(_native.load().brook_context_set_tuning(context, int(key, 16), ctypes.byref(t)))
 
@@ -81,7 +85,7 @@ def autotune(samples, teasar_params=None, anisotropy=(1, 1, 1), dust_threshold=1
     if save:
         with _lock:
             table = _read()
-            table.setdefault(_gpu_name(device), {})[f"{cls.value:x}"] = entry
+            table.setdefault(_gpu_name(device), {})[f"{cls.value:x}"] = dict(entry, engine=ENGINE)
             path = cache_path()
             os.makedirs(os.path.dirname(path), exist_ok=True)
             tmp = path + f".{os.getpid()}.tmp"
