@@ -1,6 +1,7 @@
 // The C ABI (include/brook_b200.h): argument checks, input staging into Fortran-ordered device
 // buffers, exception -> brook_status mapping with thread-local error text, result handles.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -879,10 +880,11 @@ brook_status brook_autotune(brook_context *ctx, const brook_volume *volumes, siz
       t.lone_first_percent = percent;
       consider(t);
     }
-    for (long long v : {4096LL, 32768LL}) {
+    const long long share = bk::voxel_share((long long)foreground), none = LLONG_MAX;
+    for (long long v : {share / 2, share, share + share / 2, none}) {
       bk::Tuning t = chosen;
-      t.prepare_cluster_voxels = v;
-      consider(t);
+      t.prepare_cluster_voxels = std::max(1LL, v);
+      if (t.prepare_cluster_voxels != bk::prepare_cluster_voxels((long long)foreground)) consider(t);
     }
     c.tuning[cls] = chosen;
     c.stats["autotune_ms"] = chosen_ms;

@@ -1558,12 +1558,14 @@ static long long resident_ctas() {
   return it->second;
 }
 
+long long voxel_share(long long foreground) { return foreground / resident_ctas(); }
+
 long long trace_cluster_voxels(long long foreground) {
-  return std::max(kTraceClusterFloor, foreground / resident_ctas() * 3 / 2);
+  return std::max(kTraceClusterFloor, voxel_share(foreground) * 3 / 2);
 }
 
 long long prepare_cluster_voxels(long long foreground) {
-  const long long share = foreground / resident_ctas();
+  const long long share = voxel_share(foreground);
   return std::max(kPrepareClusterFloor, share >= kPrepareWholeShare ? share : share / 2);
 }
 

@@ -129,17 +129,22 @@ int cluster_ctas(long long largest, long long foreground);
 constexpr long long kTraceClusterFloor = 32768;
 long long trace_cluster_voxels(long long foreground);
 // Preparation, whose floods have frontiers ten times as wide: the share from kPrepareWholeShare on, below it
-// half the share, at least kPrepareClusterFloor (prepare ms): 512^3 dense 17.8 from 20 k, 14.6 from 60 k, 13.0
-// from 100 k, 11.4 without; the batch 4.0 from 28 k, 3.1 from 56 k, 4.0 without; 256^3 dense 2.3 from 12 k, 2.7
-// from 20 k, 4.5 from 60 k.
+// half the share, at least kPrepareClusterFloor. Measured (prepare ms by the objects' least voxels for a cluster: half
+// the share, the share, one and a half, none): dense volumes with shares of 19 k 2.05, 2.15, 2.16, 3.53; 24 k 2.42, 2.68,
+// 2.72, 3.16; 34 k 3.50, 3.41, 2.96, 5.24; 43 k 4.18, 3.83, 3.43, 4.22; 55 k 4.79, 3.90, 3.87, 4.82; 89 k 6.97, 5.05, 5.48,
+// 5.80; 129 k 8.47, 6.37, 5.68, 5.68; batches with 40 k 3.66, 2.76, 2.29, 2.07; 62 k 4.92, 3.49, 2.88, 2.91. Half and whole
+// shares cross at about 30 k; one and a half were better than the whole by more than 2 % in 15 of 24 workloads from
+// 34 k on, and worse in 2 (by 4 and 9 %).
 constexpr long long kPrepareClusterFloor = 4096, kPrepareWholeShare = 32768;
 long long prepare_cluster_voxels(long long foreground);
+// An even share of the foreground voxels over the device's resident CTAs.
+long long voxel_share(long long foreground);
 
 // Tiny objects, below kTinyVoxels, take small CTAs, four to an SM, when a call has at least kTinyObjects of them: their
-// chains are a few dozen rounds of barriers and L2 round trips, which a CTA that fills an SM serves one object at a time.
-// They are launched after the others', in whose shadow a few of them cost nothing. Measured (prepare + trace ms, all on
-// large CTAs and with small ones of 256 threads; of 128): 32768 cubes of 6^3 26.5, 8.7, 6.1; 15625 of 8^3 19.5, 7.9, 6.5;
-// 4096 of 13^3 11.7, 6.7, 6.4; 2744 of 16^3 13.2, 9.4, 10.2; 1331 of 20^3 10.3, 9.1, 11.1; 2048 of 6^3 1.5, 0.6, 0.4.
+// chains are a few dozen rounds of barriers and L2 round trips, and a CTA that fills an SM serves one object at a time.
+// They are launched after the others, in whose shadow fewer of them cost nothing. Measured (prepare + trace ms, on
+// large CTAs, on small ones of 256 threads, of 128): 32768 cubes of 6^3 26.5, 8.7, 6.1; 15625 of 8^3 19.5, 7.9, 6.5; 4096 of
+// 13^3 11.7, 6.7, 6.4; 2744 of 16^3 13.2, 9.4, 10.2; 1331 of 20^3 10.3, 9.1, 11.1; 2048 of 6^3 1.5, 0.6, 0.4.
 constexpr int kTinyThreads = 256;
 constexpr int kTinyVoxels = 4096, kTinyObjects = 1024;
 
