@@ -156,8 +156,10 @@ int launch_prepare(const EngineArgs &a, int nbig, int cluster_ctas, cudaStream_t
 int launch_trace(const EngineArgs &a, int nbig, int cluster_ctas, int lone_percent, cudaStream_t stream);
 constexpr int kLoneFirstPercent = 10;
 // The railroad band's width in penalties of the nearest deferred voxel (EngineArgs::rail_band).
-// Measured on the 512^3 dense workload (trace ms): 0.1 69.8, 0.25 59.0, 0.5 56.1, 1 58.4, 2 60.6,
-// 4 66.8, 8 80.6, 16 117.7; narrower bands take more band ends, wider ones more re-relaxations.
+// Measured (trace ms at 0.1, 0.25, 0.5, 0.75, 1, 2, 4): 512^3 dense 30.0, 25.7, 25.5, 26.8, 28.1, 34.7, 55.4; 256^3 dense
+// 24.1, 18.3, 17.0, 16.9, 16.8, 17.9, 19.8; one arbor 64.4, 46.1, 40.0, 38.3, 38.3, 38.2, 42.1; a 48^3 request 8.8, 6.1, 5.5,
+// 5.4, 5.3, 5.1, 5.4; a batch of 16 10.1, 8.5, 8.0, 8.1, 11.5, 10.7, 19.5. Narrower bands take more band ends, wider
+// ones more re-relaxations.
 constexpr float kRailBand = 0.5f;
 // The device queries the launches above make (resident clusters per kernel), done ahead so that
 // a stream capture of the launches holds launches only.
