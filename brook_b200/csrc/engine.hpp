@@ -140,11 +140,13 @@ long long prepare_cluster_voxels(long long foreground);
 // An even share of the foreground voxels over the device's resident CTAs.
 long long voxel_share(long long foreground);
 
-// Tiny objects, below kTinyVoxels, take small CTAs, four to an SM, when a call has at least kTinyObjects of them: their
-// chains are a few dozen rounds of barriers and L2 round trips, and a CTA that fills an SM serves one object at a time.
-// They are launched after the others, in whose shadow fewer of them cost nothing. Measured (prepare + trace ms, on
-// large CTAs, on small ones of 256 threads, of 128): 32768 cubes of 6^3 26.5, 8.7, 6.1; 15625 of 8^3 19.5, 7.9, 6.5; 4096 of
-// 13^3 11.7, 6.7, 6.4; 2744 of 16^3 13.2, 9.4, 10.2; 1331 of 20^3 10.3, 9.1, 11.1; 2048 of 6^3 1.5, 0.6, 0.4.
+// Tiny objects, below kTinyVoxels, take small CTAs, four to an SM, when a call has at least kTinyObjects of them and
+// they hold half of its foreground: their chains are a few dozen rounds of barriers and L2 round trips, and a CTA that
+// fills an SM serves one object at a time. They are launched after the others, in whose shadow fewer of them cost
+// nothing (a batch of 32 volumes, 1795 objects, more than 1024 of them tiny: 20.1 in one launch, 22.2 in two). Measured
+// (prepare + trace ms, on large CTAs, on small ones of 256 threads, of 128): 32768 cubes of 6^3 26.5, 8.7, 6.1; 15625 of
+// 8^3 19.5, 7.9, 6.5; 4096 of 13^3 11.7, 6.7, 6.4; 2744 of 16^3 13.2, 9.4, 10.2; 1331 of 20^3 10.3, 9.1, 11.1; 2048 of
+// 6^3 1.5, 0.6, 0.4.
 constexpr int kTinyThreads = 256;
 constexpr int kTinyVoxels = 4096, kTinyObjects = 1024;
 

@@ -596,8 +596,13 @@ std::vector<Packed> skeletonize(Context &ctx, const std::vector<DeviceVolume> &v
   const int nbig_trace = leading("BROOK_B200_TRACE_CLUSTER_VOXELS",
                                  tune.trace_cluster_voxels > 0 ? tune.trace_cluster_voxels : trace_cluster_voxels(F));
   int ntiny = 0;
-  while (ntiny < nobj - std::max(nbig_prepare, nbig_trace) && obj_count[schedule[nobj - 1 - ntiny]] < kTinyVoxels) ++ntiny;
-  if (ntiny < kTinyObjects) ntiny = 0;
+  long long tiny_voxels = 0;
+  for (; ntiny < nobj - std::max(nbig_prepare, nbig_trace); ++ntiny) {
+    const int count = obj_count[schedule[nobj - 1 - ntiny]];
+    if (count >= kTinyVoxels) break;
+    tiny_voxels += count;
+  }
+  if (ntiny < kTinyObjects || 2 * tiny_voxels < F) ntiny = 0;
   auto d_arena_offset = to_device(ctx, arena_offset), d_arena_dims = to_device(ctx, arena_dims);
   auto d_obj_arena = to_device(ctx, obj_arena), d_obj_begin = to_device(ctx, obj_begin), d_obj_count = to_device(ctx, obj_count);
   auto d_schedule = to_device(ctx, schedule), d_border_root = to_device(ctx, border_root);

@@ -1,6 +1,6 @@
 """Calls with many tiny objects, which run on CTAs of 256 threads after the others': objects of one voxel to the 4095 that
-still count as tiny (frontiers past the small queues among them), beside larger ones, and calls just below and at the 1024
-tiny objects that call for it. Skeletons must be the oracle's bit for bit."""
+still count as tiny (frontiers past the small queues among them), beside larger ones; calls just below and at the 1024
+tiny objects that call for it, and with a larger object that holds more than they do. Skeletons must be the oracle's bit for bit."""
 import numpy as np
 import pytest
 
@@ -60,6 +60,10 @@ def test_about_as_many_tiny_objects_as_call_for_small_ctas(gpu, count):
         opts["dust_threshold"] = low
         assert_same(bk().skeletonize(labels, output="packed", **opts), oracle.skeletonize(labels, threads=8, **opts),
                     f"{count}, dust {low}")
+    opts["dust_threshold"] = 0
+    slab = np.asfortranarray(np.pad(labels, ((0, 0), (0, 0), (0, 20))))
+    slab[:, :, -18:] = 60000
+    assert_same(bk().skeletonize(slab, output="packed", **opts), oracle.skeletonize(slab, threads=8, **opts), "slab")
 
 
 def test_batch_of_tiny_and_large_objects(gpu):
