@@ -676,7 +676,7 @@ def run_ours(args, cfg):
     achieved = trace_bytes / (stage.get("ms_trace", float("nan")) / 1e3) / 1e9
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "traffic_dense512.txt")
-    if os.path.exists(tfile):
+    if cfg is CONFIGS["dense512"] and os.path.exists(tfile):  # captured on that workload
         for line in open(tfile):
             if line.startswith("trace_kernel dram_bytes_per_launch"):
                 traffic = float(line.split("=")[1])

@@ -33,10 +33,11 @@ import numpy as np
 from .batch import skeletonize_batch
 
 # Device bytes per voxel beyond the labels: component ids, neighbour masks, DBF, the per-voxel
-# engine state (PDRF, distances, DAF, flags, liveness, claim keys), union-find / scan scratch, the
+# engine state (PDRF, distances, DAF, flags, claim keys), union-find / scan scratch, the
 # EDT's envelope stacks, the per-object worklists and the allocator's size-class rounding. The
-# context's high-water marks measured 157 bytes per voxel for a 512^3 dense volume (22 % of it
-# foreground) and 142 for nine overlapping 512x512x256 chunks (44 %).
+# context's high-water marks measured 54 bytes per voxel for a 512^3 dense volume (21 % of it
+# foreground) where the EDT scans; where its spacing calls for the envelope, the stacks brought such
+# a volume to 157.
 STATE_BYTES_PER_VOXEL = 160
 # Device bytes per request that do not scale with its voxels: per-volume tables, the face stack
 # of its border targets, size-class rounding of its small buffers.

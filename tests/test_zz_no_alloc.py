@@ -72,9 +72,9 @@ def test_noalloc_edt_matches_brook_edt_twice(gpu):
 
 
 def test_noalloc_edt_over_several_stack_batches(gpu):
-    """A volume whose y and z passes need more envelope stack than the fixed scratch holds at
-    once (256 x 256 x 64: about 68 MB of y-pass stacks), so each pass runs in several batches of
-    lines over the same scratch; twice in a row, equal to brook_edt bit for bit."""
+    """A volume whose envelope stacks would not fit the fixed scratch at once (256 x 256 x 64: about
+    68 MB of y-pass stacks); twice in a row, equal to brook_edt bit for bit. At these spacings the
+    passes scan and keep no stacks; test_gpu_edt_scan's envelope test runs the batches of stacks."""
     import torch
 
     from brook_b200 import _native as n
